@@ -154,7 +154,10 @@ int lbl_line_prep_jac(const LineIn* lines, int n_lines, const LayerGroup* lg, in
  * pylblrtm/forward.py:295-315 (tile loop, _voigt, phi @ S, radiation term and
  * its finiteness check). od: [n_rows, n_nu]. evals (nullable, u64) receives
  * the number of (row, point, line) evaluations admitted by the tile rule.
- * _f64: float64 throughout (Gautschi-type Faddeeva). _f32: float32 Faddeeva
+ * _f64: float64 throughout; lines farther than six half-widths from an interval
+ * (512-, 256- or 32-point) contribute through 16 Chebyshev nodes of it, at float64
+ * accuracy, the others directly, by the asymptotic series or Weideman's 48-term
+ * approximation; fixed summation order. _f32: float32 Faddeeva
  * with the asymptotic far-wing branch and compensated sums. */
 int lbl_tau_tiles_f64(const LineF64* prep, int n_lines, const int* ranges, const double* t_layer, int n_rows,
                       double nu_min, double step, long long n_nu, int tile_samples, double cutoff, int n_grp,

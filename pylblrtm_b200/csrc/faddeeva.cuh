@@ -182,8 +182,8 @@ LBL_HD cpx<T> faddeeva(T x, T y) {
 // against scipy.special.wofz; N = 28 below (coefficients: gen_weideman.py).
 template <int N, bool HORNER = false>
 LBL_HD cpx<double> weideman_upper_n(double x, double y) {
-  static_assert(N == LBL_WEIDEMAN_N || N == LBL_WEIDEMAN28_N, "coefficient set");
-  constexpr double L = N == LBL_WEIDEMAN_N ? LBL_WEIDEMAN_L : LBL_WEIDEMAN28_L;
+  static_assert(N == LBL_WEIDEMAN_N || N == LBL_WEIDEMAN28_N || N == LBL_WEIDEMAN48_N, "coefficient set");
+  constexpr double L = N == LBL_WEIDEMAN_N ? LBL_WEIDEMAN_L : N == LBL_WEIDEMAN28_N ? LBL_WEIDEMAN28_L : LBL_WEIDEMAN48_L;
   const double dr = L + y, di = -x;             // L - i z
   const double nr = L - y, ni = x;              // L + i z
   const double inv = 1.0 / (dr * dr + di * di);
@@ -191,6 +191,9 @@ LBL_HD cpx<double> weideman_upper_n(double x, double y) {
   double a[N];                                   // folded into immediates when unrolled
   if constexpr (N == LBL_WEIDEMAN_N) {
     const double c[N] = {LBL_WEIDEMAN_COEFFS};
+    for (int k = 0; k < N; ++k) a[k] = c[k];
+  } else if constexpr (N == LBL_WEIDEMAN48_N) {
+    const double c[N] = {LBL_WEIDEMAN48_COEFFS};
     for (int k = 0; k < N; ++k) a[k] = c[k];
   } else {
     const double c[N] = {LBL_WEIDEMAN28_COEFFS};
@@ -246,6 +249,31 @@ LBL_HD double weideman_re(double x, double y) {
 LBL_HD double weideman_re_f32(double x, double y) { return weideman_re<LBL_WEIDEMAN28_N>(x, y); }
 // The same by complex Horner, for rarely taken paths of kernels at their register limit.
 LBL_HD double weideman_re_f32_compact(double x, double y) { return weideman_re<LBL_WEIDEMAN28_N, true>(x, y); }
+
+// Re w inside |z|^2 < 49 for the float64 engine: the 48-term set (against scipy.special.wofz
+// within 5e-12 of Re w for y >= 1e-3 and 5e-11 for y >= 1e-4; the Maclaurin and Taylor
+// branches of faddeeva() above reach 2e-8 and 2e-7 there).
+LBL_HD double weideman_re_f64(double x, double y) { return weideman_re<LBL_WEIDEMAN48_N>(x, y); }
+
+// Re w by N terms of the asymptotic series (i/sqrt(pi)) sum (2k-1)!!/2^k z^-(2k+1), complex
+// Horner in u = 1/z^2 = (zr + i zi)^2 with zr + i zi = 1/z. Every imaginary part carries the
+// factor y, so Re w keeps its relative accuracy for small y.
+template <int N>
+LBL_HD double re_w_series(double zr, double zi) {
+  const double ur = zr * zr - zi * zi, ui = 2.0 * zr * zi;
+  double c[N];                                   // folded into immediates when unrolled
+  c[0] = 1.0;
+#pragma unroll
+  for (int k = 1; k < N; ++k) c[k] = c[k - 1] * (k - 0.5);
+  double pr = c[N - 1], pi = 0.0;
+#pragma unroll
+  for (int k = N - 2; k >= 0; --k) {
+    const double t = fma(pr, ur, fma(-pi, ui, c[k]));
+    pi = fma(pr, ui, pi * ur);
+    pr = t;
+  }
+  return -INV_SQRT_PI * fma(zr, pi, zi * pr);
+}
 
 // |z|^2 below which the engine evaluates Re w in double precision (Weideman's
 // approximation): inside it a float complex evaluation loses relative accuracy

@@ -13,12 +13,23 @@ void lbl_host_faddeeva_f64(const double* x, const double* y, long long n, double
   }
 }
 
-// Re w by Weideman's approximation with the 36-term set (terms = 36) or the 28-term
-// set of the float32 multi-level engine's near zone (terms = 28).
+// Re w by Weideman's approximation with the 36-term set (terms = 36), the 28-term set of
+// the float32 multi-level engine's near zone (28) or the 48-term set of the float64 engine (48).
 int lbl_host_weideman_re(const double* x, const double* y, long long n, int terms, double* re) {
-  if (terms != 36 && terms != 28) return -1;
+  if (terms != 36 && terms != 28 && terms != 48) return -1;
   for (long long i = 0; i < n; ++i)
-    re[i] = terms == 36 ? lbl::weideman_re(x[i], y[i]) : lbl::weideman_re_f32(x[i], y[i]);
+    re[i] = terms == 36 ? lbl::weideman_re(x[i], y[i])
+            : terms == 28 ? lbl::weideman_re_f32(x[i], y[i]) : lbl::weideman_re_f64(x[i], y[i]);
+  return 0;
+}
+
+// Re w by the float64 engine's asymptotic series (terms = 13 or 22), y >= 0.
+int lbl_host_series_re(const double* x, const double* y, long long n, int terms, double* re) {
+  if (terms != 13 && terms != 22) return -1;
+  for (long long i = 0; i < n; ++i) {
+    const double r = 1.0 / (x[i] * x[i] + y[i] * y[i]);
+    re[i] = terms == 13 ? lbl::re_w_series<13>(x[i] * r, -y[i] * r) : lbl::re_w_series<22>(x[i] * r, -y[i] * r);
+  }
   return 0;
 }
 

@@ -16,7 +16,6 @@
 namespace lbl {
 
 constexpr int F32_P = 8;          // grid points per thread (float32 kernel)
-constexpr int F64_P = 4;          // grid points per thread (float64 kernel)
 constexpr int MAX_THREADS = 128;  // threads per CTA (and lines staged per round)
 
 struct StagedF32 {
@@ -160,70 +159,6 @@ tau_f32_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
   if (evals && tid == 0 && n_pass) atomicAdd(evals, n_pass * (unsigned long long)(c1 - c0));
 }
 
-struct StagedF64 {
-  double nuc, inv_ad, y, amp;
-};
-
-__global__ void __launch_bounds__(MAX_THREADS)
-tau_f64_kernel(const LineF64* __restrict__ prep, int n_lines, const int2* __restrict__ ranges,
-               const double* __restrict__ t_layer, double nu_min, double step, long long n_nu,
-               int tile_samples, int chunks_per_tile, double cutoff, int n_grp, double* __restrict__ od,
-               int* err, unsigned long long* evals) {
-  constexpr int P = F64_P;
-  __shared__ StagedF64 s_l[MAX_THREADS];
-  __shared__ int warp_cnt[MAX_THREADS / 32];
-
-  const int row = blockIdx.y;
-  const int tile = blockIdx.x / chunks_per_tile, chunk = blockIdx.x % chunks_per_tile;
-  const long long t0 = (long long)tile * tile_samples;
-  const long long t1 = min(t0 + (long long)tile_samples, n_nu);
-  const long long c0 = t0 + (long long)chunk * (blockDim.x * P);
-  if (c0 >= t1) return;
-  const long long c1 = min(c0 + (long long)(blockDim.x * P), t1);
-  const double wlo = __dsub_rn(grid_nu(nu_min, step, t0), cutoff);
-  const double whi = __dadd_rn(grid_nu(nu_min, step, t1 - 1), cutoff);
-  const int2 rng = ranges[tile];
-  const LineF64* lp = prep + (long long)row * n_lines;
-  const int tid = threadIdx.x;
-
-  double nu[P], acc[P];
-#pragma unroll
-  for (int m = 0; m < P; ++m) {
-    nu[m] = grid_nu(nu_min, step, min(c0 + tid * P + m, c1 - 1));
-    acc[m] = 0.0;
-  }
-  unsigned long long n_pass = 0;
-  for (int base = rng.x; base < rng.y; base += blockDim.x) {
-    const int total = stage_round<LineF64>(
-        lp, base + tid, rng.y, wlo, whi, warp_cnt, [&](int slot, const LineF64& L) {
-          s_l[slot] = StagedF64{L.nuc, L.inv_ad, L.y, L.amp};
-        });
-    n_pass += (unsigned long long)total;
-    for (int l = 0; l < total; ++l) {
-      const StagedF64 L = s_l[l];
-#pragma unroll
-      for (int m = 0; m < P; ++m) {
-        const double x = (nu[m] - L.nuc) * L.inv_ad;
-        acc[m] = fma(L.amp, re_w_f64(x, L.y), acc[m]);
-      }
-    }
-  }
-  const double T = t_layer[row];
-  double* out = od + (long long)row * n_nu;
-  bool bad = false;
-#pragma unroll
-  for (int m = 0; m < P; ++m) {
-    const long long p = c0 + tid * P + m;
-    if (p < c1) {
-      const double v = __dmul_rn(acc[m], radiation_term_grid(nu[m], T));
-      bad |= !isfinite(v);
-      out[p] = v;
-    }
-  }
-  if (bad) flag_error(err, row * (n_grp + 1) + n_grp);
-  if (evals && tid == 0 && n_pass) atomicAdd(evals, n_pass * (unsigned long long)(c1 - c0));
-}
-
 // Threads per CTA for a reference tile: enough warps for the tile, at most 128.
 static int tile_threads(int tile_samples, int points_per_thread) {
   int warps = (tile_samples + 32 * points_per_thread - 1) / (32 * points_per_thread);
@@ -298,14 +233,6 @@ extern "C" int lbl_tau_tiles_f32(const LineF32* prep, int n_lines, const int* ra
                                  void* stream) {
   return launch_tau(tau_f32_kernel, F32_P, prep, n_lines, ranges, t_layer, n_rows, nu_min, step, n_nu,
                     tile_samples, cutoff, n_grp, od, err, evals, stream, "lbl_tau_tiles_f32");
-}
-
-extern "C" int lbl_tau_tiles_f64(const LineF64* prep, int n_lines, const int* ranges, const double* t_layer,
-                                 int n_rows, double nu_min, double step, long long n_nu, int tile_samples,
-                                 double cutoff, int n_grp, double* od, int* err, unsigned long long* evals,
-                                 void* stream) {
-  return launch_tau(tau_f64_kernel, F64_P, prep, n_lines, ranges, t_layer, n_rows, nu_min, step, n_nu,
-                    tile_samples, cutoff, n_grp, od, err, evals, stream, "lbl_tau_tiles_f64");
 }
 
 template <typename T>

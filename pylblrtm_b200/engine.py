@@ -36,7 +36,7 @@ from .spectral_data import SpectralData
 
 INT_MAX = 2**31 - 1
 # "fp32": multi-level float32 summation (default); "fp32-direct": float32 summation of
-# every line at every point; "fp64": the plain float64 method.
+# every line at every point; "fp64": float64 throughout.
 PRECISIONS = ("fp32", "fp32-direct", "fp64")
 
 

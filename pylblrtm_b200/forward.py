@@ -6,7 +6,7 @@ the GPU through :mod:`pylblrtm_b200.engine`. Two engine precisions exist:
 
 * ``precision="fp32"`` (default): float32 Faddeeva with an asymptotic far-wing
   branch and compensated sums; |dT| <= 1e-5 against the float64 reference.
-* ``precision="fp64"``: float64 throughout (Gautschi-type Faddeeva);
+* ``precision="fp64"``: float64 throughout (far lines through Chebyshev nodes at float64 accuracy);
   |dT| <= 1e-6.
 """
 
