@@ -59,6 +59,22 @@ int lbl_map_index(const int* index, long long n, const int* lut, int n_lut, int*
 long long lbl_count_band(const double* nu0, const double* shift, const int* gid, long long n, double lo_edge,
                          double hi_edge, double p_max);
 
+/* lbl_line_pairs that also lists the lines inside the band mask: *n_band of them, their
+ * positions in the list (band_line) and pairs (band_pair), in input order; both arrays have
+ * room for n entries. Runs on up to eight threads of its own for long lists. */
+int lbl_band_scan(const int* mol, const int* iso, const double* nu0, const double* shift, long long n,
+                  double lo_edge, double hi_edge, double p_max, int max_pairs, int* pair_mol, int* pair_iso,
+                  long long* pair_band, int* n_pairs, int* band_line, int* band_pair, long long* n_band,
+                  double* max_abs_shift);
+
+/* Packs the listed lines of the contributing groups for the upload: for every i < n_band with
+ * lut[band_pair[i]] >= 0 and, with narrowed != 0, nu0 inside the band of lbl_count_band, the
+ * seven columns cols[0..6] (centres first, shifts last) go to out[c * stride + j] and the group to gid[j], in list order. With out = NULL only counts.
+ * Returns the number of lines kept; -1 for bad arguments or when it exceeds stride. */
+long long lbl_pack_band(const double* const* cols, const int* band_line, const int* band_pair, long long n_band,
+                        const int* lut, int n_lut, int narrowed, double lo_edge, double hi_edge, double p_max,
+                        double* out, long long stride, int* gid);
+
 #ifdef __cplusplus
 }
 #endif

@@ -91,6 +91,8 @@ HOST_SIGNATURES = {
     "lbl_par_parse": (_I, [ctypes.c_char_p, _L, _L, _P, _P, _P]),
     "lbl_line_pairs": (_I, [_P, _P, _P, _P, _L, _D, _D, _D, _I, _P, _P, _P, _P, _P, _P]),
     "lbl_map_index": (_I, [_P, _L, _P, _I, _P]),
+    "lbl_band_scan": (_I, [_P, _P, _P, _P, _L, _D, _D, _D, _I, _P, _P, _P, _P, _P, _P, _P, _P]),
+    "lbl_pack_band": (_L, [_P, _P, _P, _L, _P, _I, _I, _D, _D, _D, _P, _L, _P]),
     "lbl_count_band": (_L, [_P, _P, _P, _L, _D, _D, _D]),
 }
 

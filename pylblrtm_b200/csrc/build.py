@@ -68,7 +68,7 @@ def build_io() -> str:
     """Host (g++) build of the HITRAN reader and line scan, liblblio.so (no CUDA); no
     floating-point contraction, so host arithmetic rounds like NumPy's."""
     tmp = IO_LIB + ".tmp"
-    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-fPIC", "-shared",
+    subprocess.run(["g++", "-O3", "-std=c++17", "-ffp-contract=off", "-fPIC", "-shared", "-pthread",
                     os.path.join(HERE, "hitran_par.cpp"), os.path.join(HERE, "host_scan.cpp"), "-o", tmp],
                    check=True)
     os.replace(tmp, IO_LIB)
