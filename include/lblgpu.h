@@ -306,6 +306,10 @@ int lbl_tensor_map_bf16(void* map_out, const void* base, long long rows, long lo
  * pipeline wait timed out (the CTA's tile is then not written). */
 int lbl_gemm_bf16(const void* map_a, const void* map_b, int M, int N, int K, int n_split,
                   const LblGemmEpilogue* ep, int* err, void* stream);
+/* count products of the same shape in as few launches as fit (8 each), the networks of an
+ * ensemble: product i is A_i . B_i^T with epilogue ep[i] (no split-K, no loss). */
+int lbl_gemm_bf16_group(int count, const void* const* map_a, const void* const* map_b, int M, int N, int K,
+                        const LblGemmEpilogue* ep, int* err, void* stream);
 /* Adam (bias-corrected, step >= 1) on float32 master weights w [rows, cols] (row stride
  * ld) with moments m, v; the gradient is the in-order sum of n_split partials of g.
  * Refreshes the bf16 copy w_bf16 [rows, ld] and its transpose wt_bf16 [cols, ld_t]
@@ -313,6 +317,36 @@ int lbl_gemm_bf16(const void* map_a, const void* map_b, int M, int N, int K, int
 int lbl_adam_step(float* w, float* m, float* v, const float* g, int n_split, long long split_stride, int rows,
                   int cols, int ld, float lr, float b1, float b2, float eps, int step, void* w_bf16, void* wt_bf16,
                   int ld_t, void* stream);
+/* The same update of several contiguous tensors (16 per launch): cols a multiple of 4, rows
+ * too when wt_bf16 ([cols, rows]) is given; 16-byte aligned buffers. */
+typedef struct {
+  float* w;
+  float* m;
+  float* v;
+  const float* g;               /* n_split partials of [rows, cols], split_stride elements apart */
+  long long split_stride;
+  void* w_bf16;                 /* NULL: no bf16 copy */
+  void* wt_bf16;                /* NULL: no transposed bf16 copy */
+  int n_split, rows, cols, pad0;
+} LblAdamItem;
+int lbl_adam_group(const LblAdamItem* items, int count, float lr, float b1, float b2, float eps, int step,
+                   void* stream);
+/* out[r] = sum_c x[r, c] of several bf16 matrices (16 per launch); cols and ld multiples of 8. */
+typedef struct {
+  const void* x;                /* bf16 [rows, ld], 16-byte aligned */
+  float* out;
+  int rows, cols, ld, pad0;
+} LblRowsumItem;
+int lbl_rowsum_group(const LblRowsumItem* items, int count, void* stream);
+/* lbl_pack_inputs_bf16 of the same raw inputs for several networks (16 per launch), x only:
+ * x [rows, ld] 16-byte aligned, ld a multiple of 8. */
+typedef struct {
+  const float* mean;
+  const float* inv_std;
+  void* x;
+} LblPackItem;
+int lbl_pack_inputs_group(const float* raw, int rows, int cols, const LblPackItem* items, int count, int ld,
+                          void* stream);
 /* out[r] = sum_c x[r, c] of a bf16 matrix (bias gradients). */
 int lbl_rowsum_bf16(const void* x, int rows, int cols, int ld, float* out, void* stream);
 /* Standardised bf16 network inputs: x[b, c] = (raw[b, c] - mean[c]) * inv_std[c] for

@@ -64,6 +64,10 @@ SIGNATURES = {
     "lbl_tensor_map_bytes": (_S, []),
     "lbl_tensor_map_bf16": (_I, [_P, _P, _L, _L, _L]),
     "lbl_gemm_bf16": (_I, [_P, _P, _I, _I, _I, _I, _P, _P, _P]),
+    "lbl_gemm_bf16_group": (_I, [_I, _P, _P, _I, _I, _I, _P, _P, _P]),
+    "lbl_adam_group": (_I, [_P, _I, _F, _F, _F, _F, _I, _P]),
+    "lbl_rowsum_group": (_I, [_P, _I, _P]),
+    "lbl_pack_inputs_group": (_I, [_P, _I, _I, _P, _I, _I, _P]),
     "lbl_adam_step": (_I, [_P, _P, _P, _P, _I, _L, _I, _I, _I, _F, _F, _F, _F, _I, _P, _P, _I, _P]),
     "lbl_rowsum_bf16": (_I, [_P, _I, _I, _I, _P, _P]),
     "lbl_pack_inputs_bf16": (_I, [_P, _I, _I, _P, _P, _P, _I, _P, _I, _P]),
@@ -83,6 +87,22 @@ class GemmEpilogue(ctypes.Structure):
 
 
 SIZEOF_GEMM_EPILOGUE = 136
+
+
+class AdamItem(ctypes.Structure):
+    """LblAdamItem of include/lblgpu.h."""
+    _fields_ = [("w", _P), ("m", _P), ("v", _P), ("g", _P), ("split_stride", _L), ("w_bf16", _P), ("wt_bf16", _P),
+                ("n_split", _I), ("rows", _I), ("cols", _I), ("pad0", _I)]
+
+
+class RowsumItem(ctypes.Structure):
+    """LblRowsumItem of include/lblgpu.h."""
+    _fields_ = [("x", _P), ("out", _P), ("rows", _I), ("cols", _I), ("ld", _I), ("pad0", _I)]
+
+
+class PackItem(ctypes.Structure):
+    """LblPackItem of include/lblgpu.h."""
+    _fields_ = [("mean", _P), ("inv_std", _P), ("x", _P)]
 
 # host-side helpers (liblblio.so, include/lblio.h): no CUDA
 IO_LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "liblblio.so")

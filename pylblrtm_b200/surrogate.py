@@ -358,8 +358,6 @@ class MLP:
             ep.mode = _lib.GEMM_F32
             ep.out_f32, ep.ld_f32, ep.split_stride = ws.dw[li].data_ptr(), k, n * k
             self._gemm(ws.map_dzt[li], ws.map_xt[li], n, k, B, ep, ws, stream, n_split=s)
-            _lib.call("lbl_rowsum_bf16", ws.dzt[li].data_ptr(), n, B, B, ws.db[li].data_ptr(), stream)
-            self.launches += 1
             if li > 0:
                 ep = _lib.GemmEpilogue()
                 ep.mode = _lib.GEMM_DGELU
@@ -367,17 +365,25 @@ class MLP:
                 ep.y, ep.ld_y = ws.dz[li - 1].data_ptr(), k
                 ep.y_t, ep.ld_yt = ws.dzt[li - 1].data_ptr(), B
                 self._gemm(ws.map_dz[li], self.map_wt[li], B, k, n, ep, ws, stream)
+        items = (_lib.RowsumItem * len(self.dims))(
+            *[_lib.RowsumItem(ws.dzt[li].data_ptr(), ws.db[li].data_ptr(), n, B, B) for li, (_, n) in
+              enumerate(self.dims)])
+        _lib.call("lbl_rowsum_group", ctypes.addressof(items), len(items), stream)
+        self.launches += -(-len(items) // 16)
 
     def _adam(self, ws: _Workspace, stream, lr: float) -> None:
         self.step += 1
         b1, b2 = self.betas
+        items = []
         for li, (k, n) in enumerate(self.dims):
-            _lib.call("lbl_adam_step", self.w[li].data_ptr(), self.mw[li].data_ptr(), self.vw[li].data_ptr(),
-                      ws.dw[li].data_ptr(), ws.split[li], n * k, n, k, k, lr, b1, b2, self.eps, self.step,
-                      self.w_bf[li].data_ptr(), self.wt_bf[li].data_ptr(), n, stream)
-            _lib.call("lbl_adam_step", self.b[li].data_ptr(), self.mb[li].data_ptr(), self.vb[li].data_ptr(),
-                      ws.db[li].data_ptr(), 1, 0, 1, n, n, lr, b1, b2, self.eps, self.step, 0, 0, 0, stream)
-            self.launches += 2
+            items.append(_lib.AdamItem(self.w[li].data_ptr(), self.mw[li].data_ptr(), self.vw[li].data_ptr(),
+                                       ws.dw[li].data_ptr(), n * k, self.w_bf[li].data_ptr(),
+                                       self.wt_bf[li].data_ptr(), ws.split[li], n, k))
+            items.append(_lib.AdamItem(self.b[li].data_ptr(), self.mb[li].data_ptr(), self.vb[li].data_ptr(),
+                                       ws.db[li].data_ptr(), 0, None, None, 1, 1, n))
+        arr = (_lib.AdamItem * len(items))(*items)
+        _lib.call("lbl_adam_group", ctypes.addressof(arr), len(items), lr, b1, b2, self.eps, self.step, stream)
+        self.launches += -(-len(items) // 16)
 
     def _check(self, ws: _Workspace) -> None:
         if int(ws.err.item()) != 0:
@@ -389,13 +395,17 @@ class MLP:
         Returns the device scalar of this rank's batch mean squared error (before the
         update). Data-parallel (:meth:`data_parallel`): B is the local batch.
         """
-        torch = self.torch
-        B = raw.shape[0]
-        ws = self.workspace(B, True)
-        stream = torch.cuda.current_stream().cuda_stream
-        self.launches = 0
+        ws = self.workspace(raw.shape[0], True)
         ws.raw.copy_(raw)
         ws.target.copy_(target)
+        return self._train_staged(ws, lr, check)
+
+    def _train_staged(self, ws: _Workspace, lr: Optional[float], check: bool = False):
+        """:meth:`train_step` on the batch already in ``ws.raw`` and ``ws.target``."""
+        torch = self.torch
+        B = ws.batch
+        stream = torch.cuda.current_stream().cuda_stream
+        self.launches = 0
         ws.loss.zero_()
         self._forward(ws, stream, True)
         self._backward(ws, stream)
@@ -509,9 +519,39 @@ class GatedSurrogate:
         n_pad = net0.dims[-1][1]
         pred = torch.empty((len(self.members), Bp, n_pad), dtype=torch.float32, device=net0.dev)
         self.launches = 0
-        for m, net in enumerate(self.members):
+        nets = self.members
+        stream = torch.cuda.current_stream().cuda_stream
+        if len(nets) > 1 and len({id(n) for n in nets}) == len(nets) and len({(n.n_in, *n.dims) for n in nets}) == 1:
+            # members of one architecture: each layer of all of them in one launch, which fills
+            # the SMs for a handful of profiles and evens out the last wave of a large batch
+            x = torch.broadcast_to(raw.detach(), (B, net0.n_in)).to(device=net0.dev, dtype=torch.float32).contiguous()
+            wss = [n.workspace(Bp, False) for n in nets]
+            items = (_lib.PackItem * len(nets))(
+                *[_lib.PackItem(n.mean.data_ptr(), n.inv_std.data_ptr(), w.x[0].data_ptr()) for n, w in zip(nets, wss)])
+            _lib.call("lbl_pack_inputs_group", x.data_ptr(), B, net0.n_in, ctypes.addressof(items), len(nets),
+                      net0.dims[0][0], stream)
+            addrs = lambda maps: (ctypes.c_void_p * len(nets))(*[m.addr for m in maps])
+            for li, (k, n) in enumerate(net0.dims):
+                eps = (_lib.GemmEpilogue * len(nets))()
+                last = li == len(net0.dims) - 1
+                for m, (net, w) in enumerate(zip(nets, wss)):
+                    ep = eps[m]
+                    ep.bias = net.b[li].data_ptr()
+                    if last:
+                        ep.mode, ep.n_valid = _lib.GEMM_BIAS_SIGMOID, net.n_out
+                        ep.out_f32, ep.ld_f32 = pred.data_ptr() + 4 * m * Bp * n_pad, n
+                    else:
+                        ep.mode = _lib.GEMM_BIAS_GELU
+                        ep.y, ep.ld_y = w.x[li + 1].data_ptr(), n
+                _lib.call("lbl_gemm_bf16_group", len(nets), addrs(w.map_x[li] for w in wss),
+                          addrs(net.map_w[li] for net in nets), Bp, n, k, ctypes.addressof(eps),
+                          wss[0].err.data_ptr(), stream)
+            self.launches = -(-len(nets) // 16) + len(net0.dims) * -(-len(nets) // 8)
+            for net in nets:
+                net.launches = 1 + len(net0.dims)
+            return pred, B
+        for m, net in enumerate(nets):
             ws = net.workspace(Bp, False)
-            stream = torch.cuda.current_stream().cuda_stream
             net.launches = 0
             ws.raw[:B].copy_(raw)
             if Bp > B:
@@ -657,7 +697,17 @@ class Trainer:
             perm = self._order()
         idx = perm[self.cursor:self.cursor + cfg.batch]
         self.cursor += cfg.batch
-        return self.net.train_step(self.x[idx], self.y[idx], lr=lr_at(cfg, self.net.step))
+        net, torch = self.net, self.net.torch
+        if self.x.shape[1:] != (net.n_in,) or self.y.shape[1:] != (net.n_out,):
+            return net.train_step(self.x[idx], self.y[idx], lr=lr_at(cfg, net.step))
+        ws = net.workspace(cfg.batch, True)          # the batch is gathered where the step reads it
+        torch.index_select(self.x.detach(), 0, idx, out=ws.raw)
+        torch.index_select(self.y.detach(), 0, idx, out=ws.target)
+        return net._train_staged(ws, lr_at(cfg, net.step))
+
+    def _read_losses(self, pending) -> None:
+        if pending:                                  # one read-back for all of them
+            self.losses.extend(self.net.torch.cat(pending).tolist())
 
     def run(self, steps: Optional[int] = None, log_every: int = 0) -> List[float]:
         n = self.cfg.steps - self.net.step if steps is None else steps
@@ -665,9 +715,9 @@ class Trainer:
         for i in range(max(0, n)):
             pending.append(self.step())
             if log_every and (self.net.step % log_every == 0):
-                self.losses.extend(float(v.item()) for v in pending)
+                self._read_losses(pending)
                 pending = []
-        self.losses.extend(float(v.item()) for v in pending)
+        self._read_losses(pending)
         self.net._check(next(iter(self.net._ws.values())))
         return self.losses
 
