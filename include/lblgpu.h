@@ -132,6 +132,30 @@ int lbl_gather_lines(const double* nu0, const double* sref, const double* g_air,
 int lbl_tile_ranges(const LineIn* lines, const int* n_kept, double nu_min, double step, long long n_nu,
                     int tile_samples, double cutoff, double pad, int n_tiles, int* ranges, void* stream);
 
+/* lbl_build_layers (or given layers: levels_p = NULL) and lbl_layer_groups in one launch:
+ * the layer temperatures t_out [n_prof * n_lay] and the per-(layer, group) records out; err
+ * (nullable) is set to INT_MAX. Same values bit for bit. */
+int lbl_layer_setup(const double* levels_p, const double* levels_t, const double* levels_vmr, const double* layer_p,
+                    const double* layer_t, const double* layer_vmr, const double* layer_col, int n_prof, int n_lay,
+                    int n_gas, int n_grp, double col_factor, const int* grp_gas, const double* grp_mass,
+                    const int* tips_off, const int* tips_len, const double* tips_t, const double* tips_q,
+                    double* t_out, LayerGroup* out, int* err, void* stream);
+
+/* lbl_sort_lines and lbl_gather_lines in one call of one to four launches for up to 262,144
+ * lines: the first n_out sorted records (n_out at most n_lines rounded up to 512) and the
+ * kept count. Same records. */
+size_t lbl_sort_gather_workspace_bytes(int n_lines);
+int lbl_sort_gather(const double* nu0, const double* sref, const double* g_air, const double* g_self,
+                    const double* elow, const double* n_air, const double* shift, const int* gid, int n_lines,
+                    double mask_lo, double mask_hi, double p_max, void* workspace, size_t workspace_bytes, int n_out,
+                    LineIn* out, int* n_kept, void* stream);
+
+/* The ranges of lbl_tile_ranges and, where given, of lbl_ml_inner_ranges (inner) and
+ * lbl_jac_near_ranges (near) in one launch. Same ranges. */
+int lbl_line_ranges(const LineIn* lines, const int* n_kept, double nu_min, double step, long long n_nu,
+                    int tile_samples, double cutoff, double pad, int n_tiles, int* ranges, int* inner, int* near,
+                    void* stream);
+
 /* Per (row = profile-layer, sorted line) HITRAN scaling; replaces
  * pylblrtm/forward.py:257-292 (strength with column and 1/R(nuc), Lorentz and
  * Doppler widths, pressure shift). out: [n_rows, n_lines]. */

@@ -40,6 +40,10 @@ SIGNATURES = {
     "lbl_sort_lines": (_I, [_P, _P, _P, _I, _D, _D, _D, _P, _S, _P, _P, _P, _P]),
     "lbl_sort_lines_noalloc": (_I, [_P, _P, _P, _I, _D, _D, _D, _P, _P, _P, _P]),
     "lbl_gather_lines": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P]),
+    "lbl_layer_setup": (_I, [_P] * 7 + [_I, _I, _I, _I, _D] + [_P] * 10),
+    "lbl_sort_gather_workspace_bytes": (_S, [_I]),
+    "lbl_sort_gather": (_I, [_P] * 8 + [_I, _D, _D, _D, _P, _S, _I, _P, _P, _P]),
+    "lbl_line_ranges": (_I, [_P, _P, _D, _D, _L, _I, _D, _D, _I, _P, _P, _P, _P]),
     "lbl_tile_ranges": (_I, [_P, _P, _D, _D, _L, _I, _D, _D, _I, _P, _P]),
     "lbl_line_prep_f64": (_I, [_P, _P, _I, _P, _I, _I, _P, _P, _P]),
     "lbl_line_prep_f32": (_I, [_P, _P, _I, _P, _I, _I, _D, _D, _P, _P, _P]),

@@ -34,3 +34,7 @@ __device__ __forceinline__ void flag_error(int* err, int key) {
 // Status plumbing of the C ABI (capi.cu).
 int lbl_set_error(int code, const char* fmt, ...);
 int lbl_check_launch(const char* what);
+// How far (cm^-1) from a tile's grid values the centres of its inner lines (forward) and of
+// its 16-node level-1 lines (Jacobian) can lie, shifts apart.
+double lbl_ml_inner_reach(int tile_samples, double step);    // voigt_ml.cu
+double lbl_jac_near_reach(int tile_samples, double step);    // voigt_ml_jac.cu

@@ -862,19 +862,23 @@ tau_ml_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restr
 
 using namespace lbl;
 
+// A line is inner for a chunk of n_c points (half-width H = (n_c - 1) / 2) when its
+// grid index j0 = rint((nuc - nu_min) / step) lies within H + 1 points of the chunk,
+// so nuc lies within (H + 1.5) steps of it; chunks lie inside their tile and have at
+// most min(tile_samples, chunk size) points. Two further steps absorb rounding.
+double lbl_ml_inner_reach(int tile_samples, double step) {
+  const int per_tile = tile_samples < ML_CHUNK ? tile_samples : ML_CHUNK;
+  const int cp = 32 * ((per_tile + ML_WARP_PTS - 1) / ML_WARP_PTS) * ML_P;
+  const int n_c_max = tile_samples < cp ? tile_samples : cp;
+  return (0.5 * (n_c_max - 1) + 3.5) * step;
+}
+
 extern "C" int lbl_ml_inner_ranges(const LineIn* lines, const int* n_kept, double nu_min, double step, long long n_nu,
                                    int tile_samples, double pad, int n_tiles, int* inner, void* stream) {
   if (tile_samples < 1 || !(step > 0))
     return lbl_set_error(LBL_EINVAL, "lbl_ml_inner_ranges: bad arguments");
-  // A line is inner for a chunk of n_c points (half-width H = (n_c - 1) / 2) when its
-  // grid index j0 = rint((nuc - nu_min) / step) lies within H + 1 points of the chunk,
-  // so nuc lies within (H + 1.5) steps of it; chunks lie inside their tile and have at
-  // most min(tile_samples, chunk size) points. Two further steps absorb rounding.
-  const int per_tile = tile_samples < ML_CHUNK ? tile_samples : ML_CHUNK;
-  const int cp = 32 * ((per_tile + ML_WARP_PTS - 1) / ML_WARP_PTS) * ML_P;
-  const int n_c_max = tile_samples < cp ? tile_samples : cp;
-  const double reach = (0.5 * (n_c_max - 1) + 3.5) * step;
-  return lbl_tile_ranges(lines, n_kept, nu_min, step, n_nu, tile_samples, reach, pad, n_tiles, inner, stream);
+  return lbl_tile_ranges(lines, n_kept, nu_min, step, n_nu, tile_samples, lbl_ml_inner_reach(tile_samples, step), pad,
+                         n_tiles, inner, stream);
 }
 
 static void ml_geometry(int tile_samples, int* threads, int* cp, long long* chunks) {

@@ -847,19 +847,23 @@ extern "C" long long lbl_jacobian_ml_work_floats(int n_rows, long long n_nu, int
   return (long long)n_rows * n_tiles * chunks * MJ_NCOEF;
 }
 
+// A 16-node level-1 line of a chunk (half-width H) has |j0 - centre| <= (1 + MJ_FAR1) H, so
+// its centre lies within MJ_FAR1 H + 1.5 grid steps of the chunk; chunks lie inside their tile
+// and have at most min(tile_samples, chunk size) points. Two further steps absorb rounding.
+double lbl_jac_near_reach(int tile_samples, double step) {
+  int threads, cp;
+  long long n_all, chunks;
+  jac_geometry(tile_samples, 1, &threads, &cp, &n_all, &chunks);
+  const int n_c_max = tile_samples < cp ? tile_samples : cp;
+  return (0.5 * MJ_FAR1 * (n_c_max - 1) + 3.5) * step;
+}
+
 extern "C" int lbl_jac_near_ranges(const LineIn* lines, const int* n_kept, double nu_min, double step, long long n_nu,
                                    int tile_samples, double pad, int n_tiles, int* near, void* stream) {
   if (tile_samples < 1 || !(step > 0) || n_nu < 1)
     return lbl_set_error(LBL_EINVAL, "lbl_jac_near_ranges: bad arguments");
-  // A 16-node level-1 line of a chunk (half-width H) has |j0 - centre| <= (1 + MJ_FAR1) H, so
-  // its centre lies within MJ_FAR1 H + 1.5 grid steps of the chunk; chunks lie inside their tile
-  // and have at most min(tile_samples, chunk size) points. Two further steps absorb rounding.
-  int threads, cp;
-  long long n_all, chunks;
-  jac_geometry(tile_samples, n_nu, &threads, &cp, &n_all, &chunks);
-  const int n_c_max = tile_samples < cp ? tile_samples : cp;
-  const double reach = (0.5 * MJ_FAR1 * (n_c_max - 1) + 3.5) * step;
-  return lbl_tile_ranges(lines, n_kept, nu_min, step, n_nu, tile_samples, reach, pad, n_tiles, near, stream);
+  return lbl_tile_ranges(lines, n_kept, nu_min, step, n_nu, tile_samples, lbl_jac_near_reach(tile_samples, step), pad,
+                         n_tiles, near, stream);
 }
 
 extern "C" int lbl_jacobian_ml_f32(const LineF32* prep, const LineJac* jprep, int n_lines, const int* ranges,

@@ -25,6 +25,7 @@ import math
 import threading
 import warnings
 from dataclasses import dataclass, field
+from types import SimpleNamespace
 from typing import Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -348,14 +349,10 @@ def _upload(torch, a, dtype, device, non_blocking: bool = False):
 
 
 def sort_launches(n_lines: int) -> int:
-    """Kernels enqueued by lbl_sort_lines for n_lines (keys + bitonic stages)."""
-    n_pad = 2048
-    while n_pad < n_lines:
-        n_pad <<= 1
-    n, k = 2, 4096
-    while k <= n_pad:
-        n += (k.bit_length() - 1) - 11 + 1
-        k <<= 1
+    """Kernels enqueued by lbl_sort_gather for n_lines (block sort + merges of eight runs)."""
+    n, run = 1, 512
+    while run < n_lines:
+        n, run = n + 1, 8 * run
     return n
 
 
@@ -543,62 +540,41 @@ class Job:
         tdt = {np.dtype(np.float64): torch.float64, np.dtype(np.int32): torch.int32}
         return [dev[o:o + nb].view(tdt[dt]).reshape(sh) for o, nb, dt, sh in zip(offs, sizes, dts, shapes)]
 
-    def _device_lines(self, stream):
-        """Layers, per-(layer, group) records, band mask + sort, gather and tile ranges.
+    def _device_lines(self, stream, inner: bool = False, near: bool = False):
+        """Layers and per-(layer, group) records, band mask + sort + gather, and line ranges.
 
-        Returns (t_layer, layer_groups, lines, n_rec, ranges, n_grp): n_rec is the host's
-        bound on the kept lines, the record count of every per-line buffer (the device
+        Returns a namespace of device addresses (t_layer, lg, lines, kept, ranges, inner, near,
+        which live in ``buf``), the error word ``err`` (a tensor), n_rec and n_grp: n_rec is the
+        host's bound on the kept lines, the record count of every per-line buffer (the device
         count stays on the device).
         """
         torch, dev = self.torch, self.dev
         grid = self.grid
         n_prof, n_lay, n_nu = self.n_prof, self.n_lay, grid.n_nu
-        n_rows = n_prof * n_lay
-        n_gas = len(self.layers.gases)
-        if self.lv is not None:
-            lp, lt, lv = self.lv
-            p_atm = torch.empty((n_prof, n_lay), dtype=torch.float64, device=dev)
-            t_lay = torch.empty_like(p_atm)
-            v_lay = torch.empty((n_prof, n_gas, n_lay), dtype=torch.float64, device=dev)
-            col = torch.empty_like(v_lay)
-            _lib.call("lbl_build_layers", lp.data_ptr(), lt.data_ptr(), lv.data_ptr(), n_prof, n_lay + 1, n_gas,
-                      COLUMN_FACTOR, p_atm.data_ptr(), t_lay.data_ptr(), v_lay.data_ptr(), col.data_ptr(),
-                      stream)
-            self.launches += 1
-        else:
-            p_atm, t_lay, v_lay, col = self.lay
-        # per (layer, group)
-        n_grp = len(self.groups)
-        grp_gas, grp_mass, tips_off, tips_len, tips_t, tips_q = self.grp
-        lg = torch.empty((n_rows * n_grp * _lib.SIZEOF_LAYER_GROUP // 8,), dtype=torch.float64, device=dev)
-        _lib.call("lbl_layer_groups", t_lay.data_ptr(), p_atm.data_ptr(), v_lay.data_ptr(), col.data_ptr(),
-                  n_prof, n_lay, n_gas, n_grp, grp_gas.data_ptr(), grp_mass.data_ptr(), tips_off.data_ptr(),
-                  tips_len.data_ptr(), tips_t.data_ptr(), tips_q.data_ptr(), lg.data_ptr(), stream)
-        self.launches += 1
-        # lines: mask, sort, gather
-        d_nu0, d_sref, d_gair, d_gself, d_elow, d_nair, d_shift = self.lines_in
-        n_lines = self.n_lines
-        ws_bytes = _lib.load().lbl_sort_workspace_bytes(n_lines)
-        ws = torch.empty((ws_bytes + 7) // 8, dtype=torch.float64, device=dev)
-        order = torch.empty(n_lines, dtype=torch.int32, device=dev)
-        kept = torch.empty(1, dtype=torch.int32, device=dev)
-        max_sb = torch.empty(1, dtype=torch.float64, device=dev)
-        _lib.call("lbl_sort_lines", d_nu0.data_ptr(), d_shift.data_ptr(), self.gid.data_ptr(), n_lines,
-                  self.mask_lo, self.mask_hi, self.p_max, ws.data_ptr(), ws_bytes,
-                  order.data_ptr(), kept.data_ptr(), max_sb.data_ptr(), stream)
-        self.launches += sort_launches(n_lines)
-        self._kept = kept
-        n_kept = self.n_bound                          # >= the device's kept count
-        lines = torch.empty((n_kept * _lib.SIZEOF_LINE_IN // 8,), dtype=torch.float64, device=dev)
-        _lib.call("lbl_gather_lines", d_nu0.data_ptr(), d_sref.data_ptr(), d_gair.data_ptr(), d_gself.data_ptr(),
-                  d_elow.data_ptr(), d_nair.data_ptr(), d_shift.data_ptr(), self.gid.data_ptr(), order.data_ptr(),
-                  kept.data_ptr(), n_kept, lines.data_ptr(), stream)
+        n_rows, n_grp, n_lines, n_rec = n_prof * n_lay, len(self.groups), self.n_lines, self.n_bound
         n_tiles = (n_nu + grid.tile_samples - 1) // grid.tile_samples
-        ranges = torch.empty((n_tiles, 2), dtype=torch.int32, device=dev)
-        _lib.call("lbl_tile_ranges", lines.data_ptr(), kept.data_ptr(), grid.nu_min, grid.step, n_nu,
-                  grid.tile_samples, self.cutoff, self.pad, n_tiles, ranges.data_ptr(), stream)
-        self.launches += 2
-        return t_lay, lg, lines, n_kept, ranges, n_grp
+        ws_bytes = _lib.load().lbl_sort_gather_workspace_bytes(n_lines)
+        # one allocation for all of it, 256-byte aligned parts
+        sizes = [("t_layer", 8 * n_rows), ("lg", _lib.SIZEOF_LAYER_GROUP * n_rows * n_grp), ("ws", ws_bytes),
+                 ("kept", 4), ("lines", _lib.SIZEOF_LINE_IN * n_rec), ("ranges", 8 * n_tiles),
+                 ("inner", 8 * n_tiles if inner else 0), ("near", 8 * n_tiles if near else 0)]
+        total = sum(-(-nb // 256) * 256 for _, nb in sizes)
+        d = SimpleNamespace(buf=torch.empty(total, dtype=torch.uint8, device=dev), n_rec=n_rec, n_grp=n_grp,
+                            n_tiles=n_tiles, err=torch.empty(1, dtype=torch.int32, device=dev))
+        at = d.buf.data_ptr()
+        for name, nb in sizes:
+            setattr(d, name, at if nb else 0)
+            at += -(-nb // 256) * 256
+        lay = ([t.data_ptr() for t in self.lv] + [0] * 4) if self.lv is not None else \
+            ([0] * 3 + [t.data_ptr() for t in self.lay])
+        _lib.call("lbl_layer_setup", *lay, n_prof, n_lay, len(self.layers.gases), n_grp, COLUMN_FACTOR,
+                  *[t.data_ptr() for t in self.grp], d.t_layer, d.lg, d.err.data_ptr(), stream)
+        _lib.call("lbl_sort_gather", *[t.data_ptr() for t in self.lines_in], self.gid.data_ptr(), n_lines,
+                  self.mask_lo, self.mask_hi, self.p_max, d.ws, ws_bytes, n_rec, d.lines, d.kept, stream)
+        _lib.call("lbl_line_ranges", d.lines, d.kept, grid.nu_min, grid.step, n_nu, grid.tile_samples, self.cutoff,
+                  self.pad, n_tiles, d.ranges, d.inner, d.near, stream)
+        self.launches += 2 + sort_launches(n_lines)
+        return d
 
     def _raise_on_error(self, err, n_grp: int) -> None:
         """FloatingPointError for the first failing (layer, group) of the device error word."""
@@ -698,47 +674,40 @@ class Job:
 
         if self.empty:
             return finish(torch.zeros((n_prof, n_lay, n_nu), dtype=od_dtype, device=dev))
-        st = self._device_lines(stream)
-        if st is None:
-            return finish(torch.zeros((n_prof, n_lay, n_nu), dtype=od_dtype, device=dev))
-        t_lay, lg, lines, n_kept, ranges, n_grp = st
-        kept = self._kept
-        # per (layer, line) prep and the Voigt sums
-        err = torch.full((1,), INT_MAX, dtype=torch.int32, device=dev)
+        # "inner": lines that can be inner lines of a tile's chunks (multi-level sums)
+        d = self._device_lines(stream, inner=precision == "fp32")
+        n_kept, n_grp, err = d.n_rec, d.n_grp, d.err
+        # per (line, layer) prep and the Voigt sums
         evals = torch.zeros(4, dtype=torch.int64, device=dev) if count_evals else None
         od = torch.empty((n_prof, n_lay, n_nu), dtype=od_dtype, device=dev)
         rec = _lib.SIZEOF_LINE_F32 if single else _lib.SIZEOF_LINE_F64
         prep = torch.empty((n_rows * n_kept * rec // 8,), dtype=torch.float64, device=dev)
         self.last_prep_bytes = n_rows * n_kept * rec          # prepared line records of the summation
-        if precision == "fp32":                               # lines that can be inner lines of a tile's chunks
-            inner = torch.empty_like(ranges)
-            _lib.call("lbl_ml_inner_ranges", lines.data_ptr(), kept.data_ptr(), grid.nu_min, grid.step,
-                      grid.n_nu, grid.tile_samples, self.pad, ranges.shape[0], inner.data_ptr(), stream)
         if timer is not None:
             p0, p1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             p0.record()
             timer["prep_shape"] = (n_rows, n_kept, n_grp, rec)
         if single:
-            _lib.call("lbl_line_prep_f32", lines.data_ptr(), kept.data_ptr(), n_kept, lg.data_ptr(), n_rows, n_grp,
+            _lib.call("lbl_line_prep_f32", d.lines, d.kept, n_kept, d.lg, n_rows, n_grp,
                       grid.nu_min, grid.step, prep.data_ptr(), err.data_ptr(), stream)
         else:
-            _lib.call("lbl_line_prep_f64", lines.data_ptr(), kept.data_ptr(), n_kept, lg.data_ptr(), n_rows, n_grp,
+            _lib.call("lbl_line_prep_f64", d.lines, d.kept, n_kept, d.lg, n_rows, n_grp,
                       prep.data_ptr(), err.data_ptr(), stream)
         if timer is not None:
             p1.record()
             timer.setdefault("prep_events", []).append((p0, p1))
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
-        common = (prep.data_ptr(), n_kept, ranges.data_ptr(), t_lay.data_ptr(), n_rows, grid.nu_min, grid.step,
+        common = (prep.data_ptr(), n_kept, d.ranges, d.t_layer, n_rows, grid.nu_min, grid.step,
                   grid.n_nu, grid.tile_samples, self.cutoff, n_grp, od.data_ptr(), err.data_ptr(),
                   _lib.ptr(evals))
         if precision == "fp32":
             l1_work = torch.empty((_lib.load().lbl_ml_work_floats(n_rows, grid.tile_samples, t_count),),
                                   dtype=torch.float32, device=dev)
-            _lib.call("lbl_tau_tiles_ml_f32", common[0], common[1], common[2], inner.data_ptr(), l1_work.data_ptr(),
+            _lib.call("lbl_tau_tiles_ml_f32", common[0], common[1], common[2], d.inner, l1_work.data_ptr(),
                       *common[3:], 0 if evals is None else evals.data_ptr() + 8, t_first, t_count,
                       _lib.LBL_DETERMINISTIC if deterministic else 0, stream)
-            self.launches += 2
+            self.launches += 1
         else:
             _lib.call("lbl_tau_tiles_f32" if single else "lbl_tau_tiles_f64", *common, stream)
         if timer is not None:
@@ -778,13 +747,12 @@ def _jacobian_impl(job: Job, gas: str, g_tau=None, deterministic: bool = False):
 
     if job.empty:
         return zeros()
-    st = job._device_lines(stream)
-    if st is None:
-        return zeros()
-    t_lay, lg, lines, n_kept, ranges, n_grp = st
-    err = torch.full((1,), INT_MAX, dtype=torch.int32, device=dev)
+    # inner-line ranges of the forward's chunks (a superset for the Jacobian's smaller chunks)
+    # and the level-1 lines within four chunk half-widths
+    d = job._device_lines(stream, inner=True, near=True)
+    n_kept, n_grp, err = d.n_rec, d.n_grp, d.err
     prep = torch.empty((n_rows * n_kept * _lib.SIZEOF_LINE_F32 // 8,), dtype=torch.float64, device=dev)
-    _lib.call("lbl_line_prep_f32", lines.data_ptr(), job._kept.data_ptr(), n_kept, lg.data_ptr(), n_rows, n_grp,
+    _lib.call("lbl_line_prep_f32", d.lines, d.kept, n_kept, d.lg, n_rows, n_grp,
               grid.nu_min, grid.step, prep.data_ptr(), err.data_ptr(), stream)
     mask = 0
     for i, grp in enumerate(job.groups):
@@ -793,23 +761,15 @@ def _jacobian_impl(job: Job, gas: str, g_tau=None, deterministic: bool = False):
     _, _, tips_off, tips_len, tips_t, tips_q = job.grp
     dlnq = torch.empty((n_rows * n_grp,), dtype=torch.float64, device=dev)
     jprep = torch.empty((n_rows * n_kept * _lib.SIZEOF_LINE_JAC // 8,), dtype=torch.float64, device=dev)
-    _lib.call("lbl_line_prep_jac", lines.data_ptr(), n_kept, lg.data_ptr(), n_rows, n_grp, tips_off.data_ptr(),
+    _lib.call("lbl_line_prep_jac", d.lines, n_kept, d.lg, n_rows, n_grp, tips_off.data_ptr(),
               tips_len.data_ptr(), tips_t.data_ptr(), tips_q.data_ptr(), mask, dlnq.data_ptr(), jprep.data_ptr(),
               stream)
-    job.launches += 4
+    job.launches += 3                       # line prep and the two kernels of the Jacobian's
     flags = _lib.LBL_DETERMINISTIC if deterministic else 0
-    # inner-line ranges of the forward's chunks: a superset for the Jacobian's smaller chunks
-    inner = torch.empty_like(ranges)
-    _lib.call("lbl_ml_inner_ranges", lines.data_ptr(), job._kept.data_ptr(), grid.nu_min, grid.step, n_nu,
-              grid.tile_samples, job.pad, ranges.shape[0], inner.data_ptr(), stream)
-    near = torch.empty_like(ranges)         # level-1 lines within four chunk half-widths
-    _lib.call("lbl_jac_near_ranges", lines.data_ptr(), job._kept.data_ptr(), grid.nu_min, grid.step, n_nu,
-              grid.tile_samples, job.pad, ranges.shape[0], near.data_ptr(), stream)
     l1_work = torch.empty((_lib.load().lbl_jacobian_ml_work_floats(n_rows, n_nu, grid.tile_samples),),
                           dtype=torch.float32, device=dev)
-    job.launches += 3                       # the two range searches and the Jacobian's level-1 kernel
-    common = (prep.data_ptr(), jprep.data_ptr(), n_kept, ranges.data_ptr(), inner.data_ptr(), near.data_ptr(),
-              t_lay.data_ptr(), n_rows, n_lay, grid.nu_min, grid.step, n_nu, grid.tile_samples, job.cutoff,
+    job.launches += 2                       # the two Jacobian kernels
+    common = (prep.data_ptr(), jprep.data_ptr(), n_kept, d.ranges, d.inner, d.near, d.t_layer, n_rows, n_lay, grid.nu_min, grid.step, n_nu, grid.tile_samples, job.cutoff,
               l1_work.data_ptr())
     if g_tau is not None:
         g = torch.as_tensor(g_tau).to(device=dev, dtype=torch.float64).reshape(n_prof, n_nu).contiguous()
