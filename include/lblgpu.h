@@ -26,6 +26,7 @@ extern "C" {
 
 /* flags of the multi-level summation and Jacobian kernels */
 #define LBL_DETERMINISTIC 1   /* bit-reproducible near-zone sums (fixed order; ~10-15 % slower) */
+#define LBL_LINE_CELLS 2      /* the level-1 workspace is followed by the line cells of lbl_line_cells */
 
 /* status codes */
 #define LBL_OK 0
@@ -226,6 +227,18 @@ int lbl_tau_tiles_ml_f32(const LineF32* prep, int n_lines, const int* ranges, co
  * (16 + 8 level-1 coefficients per chunk and row); -1 for bad arguments. No reference
  * counterpart: a workspace of the summation. */
 long long lbl_ml_work_floats(int n_rows, int tile_samples, int tile_count);
+
+/* Line cells of lbl_tau_tiles_ml_f32 (no reference counterpart: a workspace of the
+ * summation): the prepared lines are cut into cells of a quarter chunk along the grid, and
+ * every (row, cell) gets the moments of its lines' far wings, so that the level-1 kernel
+ * evaluates a distant cell instead of each of its lines. lbl_line_cells_floats gives their
+ * size (0: this geometry uses none; -1: bad arguments); a caller that uses them places them
+ * behind the level-1 coefficients, at l1_work + lbl_ml_work_floats(...) rounded up to a
+ * multiple of 4 (l1_work 16-byte aligned), fills them with lbl_line_cells after
+ * lbl_line_prep_f32 and passes LBL_LINE_CELLS. */
+long long lbl_line_cells_floats(int n_rows, long long n_nu, int tile_samples, double step, double cutoff);
+int lbl_line_cells(const LineIn* lines, const int* n_kept, const LineF32* prep, int n_lines, int n_rows, double nu_min,
+                   double step, long long n_nu, int tile_samples, double cutoff, float* cells, void* stream);
 
 /* Layer Jacobians by the multi-level float32 summation (no reference
  * counterpart; the retrieval adjoint): writes od (as lbl_tau_tiles_ml_f32),

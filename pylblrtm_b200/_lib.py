@@ -14,6 +14,7 @@ import threading
 LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "liblblgpu.so")
 
 LBL_OK = 0
+LBL_LINE_CELLS = 2       # flag: line cells follow the level-1 workspace
 LBL_DETERMINISTIC = 1    # flag of the multi-level summation and Jacobian kernels
 
 # byte sizes of the records declared in include/lblgpu.h
@@ -52,6 +53,8 @@ SIGNATURES = {
     "lbl_ml_inner_ranges": (_I, [_P, _P, _D, _D, _L, _I, _D, _I, _P, _P]),
     "lbl_tau_tiles_ml_f32": (_I, [_P, _I, _P, _P, _P, _P, _I, _D, _D, _L, _I, _D, _I, _P, _P, _P, _P, _I, _I, _I,
                                   _P]),
+    "lbl_line_cells_floats": (_L, [_I, _L, _I, _D, _D]),
+    "lbl_line_cells": (_I, [_P, _P, _P, _I, _I, _D, _D, _L, _I, _D, _P, _P]),
     "lbl_ml_work_floats": (_L, [_I, _I, _I]),
     "lbl_line_prep_jac": (_I, [_P, _I, _P, _I, _I, _P, _P, _P, _P, _I, _P, _P, _P]),
     "lbl_jacobian_ml_f32": (_I, [_P, _P, _I, _P, _P, _P, _P, _I, _I, _D, _D, _L, _I, _D, _P, _P, _P, _P, _P, _P,

@@ -112,18 +112,32 @@ __device__ __forceinline__ LineJac line_jac_from_planes(const float4& p0, const 
   return J;
 }
 
-// Adds the lanes' float node sums into the warp's float64 sums (lane 0 owns the row)
-// and clears them; every lane of the warp calls it.
+// Adds the lanes' float node sums into the warp's float64 sums and clears them; every lane of
+// the warp calls it. K = 16 or 8. The sums are formed in float64 by a transposed reduction
+// (32 or 18 shuffles where a reduction per node took 160 or 80; the flush had been half of the
+// level-1 kernel's instructions once most of its lines went through cells).
 template <int K>
 __device__ __forceinline__ void flush_nodes(float (&f)[K], double* row, int lane) {
+  static_assert(K == 16 || K == 8, "node counts");
+  constexpr unsigned full = 0xffffffffu;
+  double g[K / 2];
+  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4, b1 = lane & 2;
 #pragma unroll
-  for (int k = 0; k < K; ++k) {
-    double v = (double)f[k];
+  for (int k = 0; k < K / 2; ++k)
+    g[k] = (double)(b4 ? f[k + K / 2] : f[k]) + __shfl_xor_sync(full, (double)(b4 ? f[k] : f[k + K / 2]), 16);
 #pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) row[k] += v;
-    f[k] = 0.f;
-  }
+  for (int k = 0; k < K / 4; ++k) g[k] = (b3 ? g[k + K / 4] : g[k]) + __shfl_xor_sync(full, b3 ? g[k] : g[k + K / 4], 8);
+#pragma unroll
+  for (int k = 0; k < K / 8; ++k) g[k] = (b2 ? g[k + K / 8] : g[k]) + __shfl_xor_sync(full, b2 ? g[k] : g[k + K / 8], 4);
+  double v;
+  if constexpr (K == 16) v = (b1 ? g[1] : g[0]) + __shfl_xor_sync(full, b1 ? g[0] : g[1], 2);
+  else v = g[0] + __shfl_xor_sync(full, g[0], 2);
+  v += __shfl_xor_sync(full, v, 1);
+  constexpr int per = 32 / K;                                  // lanes per node
+  if (lane % per == 0) row[lane / per] += v;
+#pragma unroll
+  for (int k = 0; k < K; ++k) f[k] = 0.f;
+  __syncwarp(full);
 }
 
 static __device__ __noinline__ float re_w_f32_mid(float x, float y, float y2, float z2) {

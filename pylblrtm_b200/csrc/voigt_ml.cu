@@ -133,16 +133,151 @@ __device__ __forceinline__ float clenshaw16(const float* c, float t) {
 }
 
 // ---------------------------------------------------------------------------
-// Level 1 as its own kernel. Nine in ten lines of a chunk's window are level-1
-// lines; each contributes only through the chunk's Chebyshev nodes, so one thread
-// takes one line and evaluates it at all nodes from registers (each thread copies its
-// own records through a cp.async ring; no barriers). The kernel leaves the chunk's
-// 16 + 8 Chebyshev coefficients in l1_work ([row][chunk of the launch][24]), which
+// Line cells: the far wings of many lines at once. The sorted lines are cut at every wp-th
+// grid point into cells; for every (row, cell) line_moments_kernel sums ten-odd real moments
+// of the lines about the cell's centre, from which tau_far_kernel gets the cell's field at a
+// far node by one polynomial instead of one evaluation per line.
+//
+// In points, with delta = node - line centre, g = y / a, w's two leading terms give
+//   amp Re w = (amp / sqrt(pi)) [ (1/a) Im 1/(delta - ig) + (1/(2a^3)) Im 1/(delta - ig)^3 ],
+// the far-wing form of far_wing_add. With D = node - cell centre and zeta = e + ig (e = line -
+// cell centre), 1/(D - zeta) = sum zeta^k / D^(k+1) and 1/(D - zeta)^3 = sum C(k,2) zeta^(k-2) /
+// D^(k+1). D is real, so only the imaginary parts count: Im zeta^k = g J_k with real J_k, and
+//   field = sum_k m_k / D^(k+1),  m_k = sum_lines (amp_far / a^2) [J_k + C(k,2) J_(k-2) / (2a^2)].
+// All in units of the cell's half-width s: field = (1/D^2) sum_k m'_k t^(k-1), t = s / D. A cell
+// is used for |zeta| / |D| <= CELL_RATIO, where the first omitted term is below 12 CELL_RATIO^11
+// ~ 1e-8 of the cell's field; nothing cancels that the lines' own rounding would not show.
+constexpr int CELL_M = 11;                     // moments k = 1 .. 11
+constexpr int CELL_F = 16;                     // floats per record: moments, g_max, e_min, e_max, a_min, lines
+constexpr float CELL_RATIO = 1.0f / 6.5f;
+constexpr int CELL_MIN = 4;                    // fewer lines are cheaper one by one
+constexpr int CELL_MIN_CHUNKS = 16;            // fewer chunks on the grid: no cells
+constexpr int CELL_MIN_PTS = 64;               // smallest cell (bounds the records to 1 byte per point and row)
+
+struct CellGeom {
+  int wp, n;            // points per cell, cells (0: none)
+  long long off;        // cell q starts at grid index q * wp - off
+};
+
+// A quarter of a chunk per cell: far cells (beyond four half-widths) then have |zeta| / |D| of
+// about 1/13. No cells where no line can be that far, for chunks shorter than two cells, or
+// for a grid of few chunks (each cell serves them all). The rule looks at the grid alone, so
+// a shard or a batch of profiles takes the same cells as the full job.
+static CellGeom cell_geometry(long long n_nu, int tile_samples, double step, double cutoff) {
+  const long long nch = (tile_samples + ML_CHUNK - 1) / ML_CHUNK;
+  const long long n_c = tile_samples / nch;
+  CellGeom g = {0, 0, 0};
+  const double reach = cutoff / step;
+  if (n_c < 2 * CELL_MIN_PTS || !(reach > 2.0 * (double)n_c) || reach > 1.0e9 ||
+      (n_nu + tile_samples - 1) / tile_samples * nch < CELL_MIN_CHUNKS)
+    return g;
+  g.wp = (int)(n_c / 4 > CELL_MIN_PTS ? n_c / 4 : CELL_MIN_PTS);
+  g.off = ((long long)reach / g.wp + 2) * g.wp;
+  const long long n = (n_nu + 2 * g.off + g.wp - 1) / g.wp;
+  if (n > 0x3fffffff) return CellGeom{0, 0, 0};
+  g.n = (int)n;
+  return g;
+}
+
+// idx[q] = first sorted line whose unshifted centre is at or beyond the start of cell q (q <= n).
+__global__ void cell_bounds_kernel(const LineIn* __restrict__ lines, const int* __restrict__ n_kept, double nu_min,
+                                   double step, CellGeom cg, int* __restrict__ idx) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q > cg.n) return;
+  const double x = grid_nu(nu_min, step, (long long)q * cg.wp - cg.off);
+  int a = 0, b = *n_kept;
+  while (a < b) {
+    const int m = (a + b) >> 1;
+    if (lines[m].nu0 < x) a = m + 1; else b = m;
+  }
+  idx[q] = a;
+}
+
+__device__ __forceinline__ float reduce16_transposed(const float (&f)[ML_K], int lane);
+
+// One warp per (cell, row).
+__global__ void __launch_bounds__(256)
+line_moments_kernel(const LineF32* __restrict__ prep, int n_lines, const int* __restrict__ idx, CellGeom cg,
+                    float* __restrict__ rec) {
+  const int q = blockIdx.x * 8 + (threadIdx.x >> 5), row = blockIdx.y, lane = threadIdx.x & 31;
+  if (q >= cg.n) return;
+  float* out = rec + ((long long)row * cg.n + q) * CELL_F;
+  const int i0 = idx[q], i1 = idx[q + 1];
+  if (i1 <= i0) {                                      // empty: only the count is read
+    if (lane == 0) out[CELL_F - 1] = 0.f;
+    return;
+  }
+  const LineF32* lp = prep + (long long)row * n_lines;
+  const int jb = (int)((long long)q * cg.wp - cg.off);
+  const float half = 0.5f * (float)cg.wp, inv_s = 1.0f / half;
+  float m[ML_K];
+#pragma unroll
+  for (int k = 0; k < ML_K; ++k) m[k] = 0.f;
+  float e_min = 3.0e38f, e_max = -3.0e38f, a_min = 3.0e38f, g_max = 0.f;
+  int cnt = 0;
+  bool ok = true;
+  for (int li = i0 + lane; li < i1; li += 32) {
+    const LineF32 L = lp[li];
+    if (!(L.nuc == L.nuc)) continue;                   // inactive
+    ++cnt;
+    const float inv_a = 1.0f / L.a;
+    const float e = (float)(L.j0 - jb) - half + L.b * inv_a, g = L.y * inv_a;
+    ok = ok && L.y >= 0.f && L.a > 0.f && g <= half;   // broad lines (or a negative width): line by line
+    e_min = fminf(e_min, e);
+    e_max = fmaxf(e_max, e);
+    a_min = fminf(a_min, L.a);
+    g_max = fmaxf(g_max, g);
+    const float zr = e * inv_s, zi = g * inv_s, nzi2 = -zi * zi;
+    const float w = L.amp_far * inv_a * inv_a, c3 = 0.5f * (inv_a * inv_s) * (inv_a * inv_s);
+    float R = zr, J = 1.0f, J1 = 0.f, J2 = 0.f;        // J = J_k, J1 = J_(k-1), J2 = J_(k-2)
+#pragma unroll
+    for (int k = 1; k <= CELL_M; ++k) {
+      const float c = 0.5f * (float)(k * (k - 1));     // C(k, 2)
+      m[k - 1] = fmaf(w, k >= 3 ? fmaf(c * c3, J2, J) : J, m[k - 1]);
+      const float Rn = fmaf(R, zr, nzi2 * J), Jn = fmaf(J, zr, R);
+      J2 = J1;
+      J1 = J;
+      R = Rn;
+      J = Jn;
+    }
+  }
+  const float v = reduce16_transposed(m, lane);        // lanes 2j, 2j + 1: moment j + 1
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    e_min = fminf(e_min, __shfl_xor_sync(0xffffffffu, e_min, o));
+    e_max = fmaxf(e_max, __shfl_xor_sync(0xffffffffu, e_max, o));
+    a_min = fminf(a_min, __shfl_xor_sync(0xffffffffu, a_min, o));
+    g_max = fmaxf(g_max, __shfl_xor_sync(0xffffffffu, g_max, o));
+  }
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  ok = __all_sync(0xffffffffu, ok);
+  if (!(lane & 1) && (lane >> 1) < CELL_M) out[lane >> 1] = v;
+  if (lane == 1) {
+    out[CELL_M] = g_max;
+    out[CELL_M + 1] = e_min;
+    out[CELL_M + 2] = e_max;
+    out[CELL_M + 3] = a_min;
+    out[CELL_M + 4] = ok ? (float)cnt : -1.f;          // counts stay far below 2^24
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Level 1 as its own kernel. Nine in ten lines of a chunk's window are level-1 lines, most of
+// them beyond four half-widths: those come as line cells (above), one thread per (cell, node).
+// Of the other level-1 lines one thread takes one and evaluates it at all nodes from
+// registers (each thread copies its own records through a cp.async ring). The kernel leaves
+// the chunk's 16 + 8 Chebyshev coefficients in l1_work ([row][chunk of the launch][24]), which
 // tau_ml_kernel reads.
-constexpr int MF_THREADS = 256;                // lines per round
+// Latency-bound: a chunk needs ~5,000 warp instructions between a handful of dependent
+// loads, so small CTAs, sixteen to an SM, cover each other's waits. Whole spectrum (200,000
+// lines, 60 layers, 950 tiles) on B200: every line by itself 1,764 us; with cells 1,209, with
+// the transposed flush 1,001, and with CTAs of 128 and 64 instead of 256 threads 688 and 610 us
+// (plus 125 us for the moments, which read the 384 MB of records once).
+constexpr int MF_THREADS = 64;                 // lines per round
 constexpr int MF_FLUSH = 32;                   // rounds summed in float before the double sums
 
 constexpr int MF_STAGES = 3;                   // rounds of line records in flight per thread
+constexpr int MF_CELLS = 512;                  // most cells of a tile's window (more: every line by itself)
 
 // amp * Re w by the far-wing form (amp_far = amp y / sqrt(pi)), added to f (|z|^2 >= FAR_Z2, y >= 0).
 __device__ __forceinline__ void far_wing_add(float& f, float x, float y2, float ny2, float amp_far) {
@@ -182,17 +317,19 @@ __device__ __forceinline__ void far_line_nodes(float (&f)[K], const float (&xs)[
   }
 }
 
-__global__ void __launch_bounds__(MF_THREADS, 4)
+__global__ void __launch_bounds__(MF_THREADS, 16)
 tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restrict__ ranges, double nu_min,
                double step, long long n_nu, int tile_samples, int chunks_per_tile, int chunk_pts, double cutoff,
-               float* __restrict__ l1_work, unsigned long long* evals, unsigned long long* work, int tile_first) {
-  // Whole 32-B records: read back by their own thread they meet 2-way bank conflicts, but
-  // the 16-B planes that jac_far_kernel stages its records in (no conflicts) made this
-  // kernel slower (summation call 10.40 -> 11.06 ms, with more spilled registers).
+               float* __restrict__ l1_work, unsigned long long* evals, unsigned long long* work, int tile_first,
+               CellGeom cg, const int* __restrict__ cell_idx, const float* __restrict__ cell_rec) {
   __shared__ __align__(16) LineF32 s_line[MF_STAGES][MF_THREADS];   // records are 32 B, 16-B aligned
   __shared__ double s_part[MF_THREADS / 32][ML_K + ML_KF];
   __shared__ float s_coef[ML_K + ML_KF];
-  __shared__ unsigned s_cnt[2];
+  __shared__ unsigned s_cnt[3];
+  __shared__ int s_use[MF_CELLS];                          // cells evaluated through their moments
+  __shared__ int s_dir[MF_CELLS], s_pre[MF_CELLS + 1];     // stretches of other lines: start, lines before
+  __shared__ int s_wu[MF_THREADS / 32], s_wd[MF_THREADS / 32], s_wl[MF_THREADS / 32];   // per-warp scan totals
+  __shared__ float s_cell[MF_THREADS / 32][ML_KF];
 
   const int row = blockIdx.y;
   const int tile = tile_first + (int)(blockIdx.x / chunks_per_tile), chunk = blockIdx.x % chunks_per_tile;
@@ -209,9 +346,8 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
   const int2 rng = ranges[tile];
   const LineF32* lp = prep + (long long)row * n_lines;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid < 2) s_cnt[tid] = 0u;
-  if (lane == 0)                                           // this warp's node sums: lane 0 alone
-    for (int k = 0; k < ML_K + ML_KF; ++k) s_part[warp][k] = 0.0;   // writes and reads them
+  if (tid < 3) s_cnt[tid] = 0u;
+  if (lane < ML_K + ML_KF) s_part[warp][lane] = 0.0;        // this warp's node sums
 
   float xa[ML_K / 2], xb[ML_KF / 2];                      // node offsets, as tau_ml_kernel places them
 #pragma unroll
@@ -226,13 +362,131 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
   for (int k = 0; k < ML_KF; ++k) ff[k] = 0.f;
   unsigned n1 = 0, nf = 0;
 
-  // line records of round r (line rng.x + r * MF_THREADS + tid) go to stage r % MF_STAGES,
-  // MF_STAGES - 1 rounds ahead; every round commits one group (empty past the end), so
-  // waiting for all but the newest MF_STAGES - 1 groups completes the current round's copy
-  const int n_rounds = rng.y > rng.x ? (rng.y - rng.x + MF_THREADS - 1) / MF_THREADS : 0;
+  // ---- the tile's lines split into cells to evaluate by their moments and other lines
+  int n_use = 0, n_dir = 1, n_direct = max(0, rng.y - rng.x);
+  if (cg.n > 0 && n_direct > 0) {
+    // the window in cells, with two cells on either side for shifted lines (checked below)
+    const double win0 = cutoff / step;
+    const int qa = (int)max(0LL, (t0 - (long long)win0 + cg.off) / cg.wp - 3);
+    const int qe = (int)min((long long)cg.n, (t1 + (long long)win0 + cg.off) / cg.wp + 3);
+    if (qe - qa <= MF_CELLS && cell_idx[qa] <= rng.x && cell_idx[qe] >= rng.y) {
+      const float* rr = cell_rec + (long long)row * cg.n * CELL_F;
+      const double wl = (double)(t0 - c0) - win0 + 1.0, wr = (double)(t1 - 1 - c0) + win0 - 1.0;   // a point of margin
+      const float half = 0.5f * (float)cg.wp;
+      n_dir = 0;
+      n_direct = 0;
+      for (int q0 = qa; q0 < qe; q0 += MF_THREADS) {
+        const int q = q0 + tid;
+        int i0 = 0, len = 0;
+        bool use = false;
+        if (q < qe) {
+          const int a = cell_idx[q], b = cell_idx[q + 1];
+          i0 = max(a, rng.x);
+          len = max(0, min(b, rng.y) - i0);
+          if (len > 0) {
+            const float4 m = *reinterpret_cast<const float4*>(rr + (long long)q * CELL_F + CELL_F - 4);
+            const float g_max = rr[(long long)q * CELL_F + CELL_M];
+            if (m.w == 0.f) len = 0;                       // only inactive lines
+            const float pc = (float)((long long)q * cg.wp - cg.off - c0) + half;
+            const float lo = pc + m.x, hi = pc + m.y;
+            // all lines beyond four half-widths on one side, inside the window, in the far-wing
+            // regime at the nearest node and well inside the series' radius
+            const float gap = fmaxf(lo - (C1 + H1), (C1 - H1) - hi);
+            const float z = fmaxf(fabsf(m.x), fabsf(m.y)) + g_max, D = fabsf(pc - C1) - H1;
+            use = m.w >= (float)CELL_MIN && i0 == a && len == b - a && gap > ML_FAR1 * H1 + 2.f && (double)lo >= wl &&
+                  (double)hi <= wr && m.z * gap >= 50.f && z <= CELL_RATIO * D;
+          }
+        }
+        const unsigned bu = __ballot_sync(0xffffffffu, use), bd = __ballot_sync(0xffffffffu, len > 0 && !use);
+        int pl = len > 0 && !use ? len : 0;                // inclusive scan of the other lines
+        const int own = pl;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int u = __shfl_up_sync(0xffffffffu, pl, o);
+          if (lane >= o) pl += u;
+        }
+        if (lane == 31) {
+          s_wu[warp] = __popc(bu);
+          s_wd[warp] = __popc(bd);
+          s_wl[warp] = pl;
+        }
+        __syncthreads();
+        int ou = n_use, od = n_dir, ol = n_direct;
+        for (int w = 0; w < MF_THREADS / 32; ++w) {
+          if (w < warp) {
+            ou += s_wu[w];
+            od += s_wd[w];
+            ol += s_wl[w];
+          }
+          n_use += s_wu[w];
+          n_dir += s_wd[w];
+          n_direct += s_wl[w];
+        }
+        const unsigned lt = (1u << lane) - 1u;
+        if (use) s_use[ou + __popc(bu & lt)] = q;
+        if (own > 0) {
+          const int o = od + __popc(bd & lt);
+          s_dir[o] = i0;
+          s_pre[o] = ol + pl - own;
+        }
+        __syncthreads();
+      }
+      if (tid == 0) s_pre[n_dir] = n_direct;
+    }
+  }
+  const bool cells = n_use > 0;
+  const bool split = cg.n > 0 && !(n_dir == 1 && n_direct == rng.y - rng.x && !cells);
+  __syncthreads();
+  if (cells) {                                             // thread: node tid % 8 of cells tid / 8, + 32, ...
+    const int k = tid & (ML_KF - 1);
+    const float xk = k < ML_KF / 2 ? H1 * c_node8[k] : -H1 * c_node8[ML_KF - 1 - k];
+    const float* rr = cell_rec + (long long)row * cg.n * CELL_F;
+    const float half = 0.5f * (float)cg.wp;
+    float f = 0.f;
+    unsigned c = 0;
+#pragma unroll 4
+    for (int i = tid >> 3; i < n_use; i += MF_THREADS / 8) {
+      const int q = s_use[i];
+      const float4* r4 = reinterpret_cast<const float4*>(rr + (long long)q * CELL_F);
+      const float4 a = r4[0], b = r4[1], d = r4[2];
+      if (k == 0) c += (unsigned)rr[(long long)q * CELL_F + CELL_F - 1];
+      const float D = (C1 + xk) - ((float)((long long)q * cg.wp - cg.off - c0) + half);
+      const float rD = 1.0f / D, t = half * rD;
+      float v = fmaf(d.z, t, d.y);
+      v = fmaf(v, t, d.x);
+      v = fmaf(v, t, b.w);
+      v = fmaf(v, t, b.z);
+      v = fmaf(v, t, b.y);
+      v = fmaf(v, t, b.x);
+      v = fmaf(v, t, a.w);
+      v = fmaf(v, t, a.z);
+      v = fmaf(v, t, a.y);
+      v = fmaf(v, t, a.x);
+      f = fmaf(rD * rD, v, f);
+    }
+    f += __shfl_xor_sync(0xffffffffu, f, 8);
+    f += __shfl_xor_sync(0xffffffffu, f, 16);
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane < ML_KF) s_cell[warp][lane] = f;
+    if (lane == 0) atomicAdd(&s_cnt[2], c);
+  }
+
+  // line records of round r (the r * MF_THREADS + tid-th of the other lines) go to stage
+  // r % MF_STAGES, MF_STAGES - 1 rounds ahead; every round commits one group (empty past the
+  // end), so waiting for all but the newest MF_STAGES - 1 groups completes the current copy
+  const int n_rounds = (n_direct + MF_THREADS - 1) / MF_THREADS;
   auto issue = [&](int r, int stage) {
-    const int li = rng.x + r * MF_THREADS + tid;
-    if (li < rng.y) {   // prep records: 32 B each in a 256-B aligned allocation
+    const int slot = r * MF_THREADS + tid;
+    if (slot < n_direct) {   // prep records: 32 B each in a 256-B aligned allocation
+      int li = rng.x + slot;
+      if (split) {           // the stretch that holds this slot
+        int a = 0, b = n_dir - 1;
+        while (a < b) {
+          const int m = (a + b + 1) >> 1;
+          if (s_pre[m] <= slot) a = m; else b = m - 1;
+        }
+        li = s_dir[a] + (slot - s_pre[a]);
+      }
       const float4* g = reinterpret_cast<const float4*>(lp + li);
       float4* d = reinterpret_cast<float4*>(&s_line[stage][tid]);
       cp_async16(d, g);
@@ -246,7 +500,7 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
   for (int r = 0; r < n_rounds; ++r) {
     issue(r + MF_STAGES - 1, stage == 0 ? MF_STAGES - 1 : stage - 1);   // the stage read last round
     cp_async_wait<MF_STAGES - 1>();
-    const bool have = rng.x + r * MF_THREADS + tid < rng.y;
+    const bool have = r * MF_THREADS + tid < n_direct;
     LineF32 L;
     if (have) L = s_line[stage][tid];
     stage = stage + 1 == MF_STAGES ? 0 : stage + 1;
@@ -288,6 +542,8 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
   if (tid < ML_K + ML_KF) {                                // column tid: only this thread touches it
     double s = 0.0;
     for (int w = 0; w < MF_THREADS / 32; ++w) s += s_part[w][tid];
+    if (cells && tid >= ML_K)
+      for (int w = 0; w < MF_THREADS / 32; ++w) s += (double)s_cell[w][tid - ML_K];
     s_part[0][tid] = s;
   }
   __syncthreads();
@@ -305,9 +561,10 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
   }
   if (tid < ML_K + ML_KF) l1_work[((long long)row * gridDim.x + blockIdx.x) * (ML_K + ML_KF) + tid] = s_coef[tid];
   if (tid == 0) {
-    const unsigned long long a = s_cnt[0], b = s_cnt[1];
-    if (evals && a + b) atomicAdd(evals, (a + b) * (unsigned long long)n_c);
-    if (work && a + b) atomicAdd(&work[0], a * ML_K + b * ML_KF);
+    const unsigned long long a = s_cnt[0], b = s_cnt[1], c = s_cnt[2];
+    if (evals && a + b + c) atomicAdd(evals, (a + b + c) * (unsigned long long)n_c);
+    // a cell at a node costs about two line evaluations
+    if (work && a + b + c) atomicAdd(&work[0], a * ML_K + b * ML_KF + 2ull * n_use * ML_KF);
   }
 }
 
@@ -896,6 +1153,30 @@ extern "C" long long lbl_ml_work_floats(int n_rows, int tile_samples, int tile_c
   return (long long)n_rows * tile_count * chunks * (ML_K + ML_KF);
 }
 
+// Layout of the line cells: cell bounds (int, n + 1, padded to 4), then the records.
+static long long cell_head(const CellGeom& g) { return ((long long)g.n + 1 + 3) / 4 * 4; }
+
+extern "C" long long lbl_line_cells_floats(int n_rows, long long n_nu, int tile_samples, double step, double cutoff) {
+  if (n_rows < 1 || n_nu < 1 || tile_samples < 1 || !(step > 0) || !(cutoff >= 0)) return -1;
+  const CellGeom g = cell_geometry(n_nu, tile_samples, step, cutoff);
+  return g.n == 0 ? 0 : cell_head(g) + (long long)n_rows * g.n * CELL_F;
+}
+
+extern "C" int lbl_line_cells(const LineIn* lines, const int* n_kept, const LineF32* prep, int n_lines, int n_rows,
+                              double nu_min, double step, long long n_nu, int tile_samples, double cutoff, float* cells,
+                              void* stream) {
+  if (!lines || !n_kept || !prep || !cells || n_lines < 1 || n_rows < 1 || n_rows > 65535 || n_nu < 1 ||
+      tile_samples < 1 || !(step > 0) || !(cutoff >= 0) || ((uintptr_t)cells) % 16)
+    return lbl_set_error(LBL_EINVAL, "lbl_line_cells: bad arguments");
+  const CellGeom g = cell_geometry(n_nu, tile_samples, step, cutoff);
+  if (g.n == 0) return LBL_OK;
+  const cudaStream_t st = (cudaStream_t)stream;
+  cell_bounds_kernel<<<g.n / 128 + 1, 128, 0, st>>>(lines, n_kept, nu_min, step, g, (int*)cells);
+  dim3 grid((unsigned)((g.n + 7) / 8), (unsigned)n_rows);
+  line_moments_kernel<<<grid, 256, 0, st>>>(prep, n_lines, (const int*)cells, g, cells + cell_head(g));
+  return lbl_check_launch("lbl_line_cells");
+}
+
 extern "C" int lbl_tau_tiles_ml_f32(const LineF32* prep, int n_lines, const int* ranges, const int* inner,
                                     float* l1_work, const double* t_layer, int n_rows, double nu_min, double step,
                                     long long n_nu, int tile_samples, double cutoff, int n_grp, float* od, int* err,
@@ -919,8 +1200,18 @@ extern "C" int lbl_tau_tiles_ml_f32(const LineF32* prep, int n_lines, const int*
   if (n_tiles * chunks * parts > 0x7fffffffLL) return lbl_set_error(LBL_EINVAL, "lbl_tau_tiles_ml_f32: grid too large");
   dim3 grid_far((unsigned)(n_tiles * chunks), (unsigned)n_rows);
   cudaStream_t st = (cudaStream_t)stream;
+  // with LBL_LINE_CELLS the line cells follow the level-1 coefficients (16-byte aligned)
+  CellGeom cg = {0, 0, 0};
+  const float* cells = nullptr;
+  if (flags & LBL_LINE_CELLS) {
+    cg = cell_geometry(n_nu, tile_samples, step, cutoff);
+    cells = l1_work + ((long long)n_rows * n_tiles * chunks * (ML_K + ML_KF) + 3) / 4 * 4;
+    if (((uintptr_t)l1_work) % 16)
+      return lbl_set_error(LBL_EINVAL, "lbl_tau_tiles_ml_f32: l1_work must be 16-byte aligned");
+  }
   tau_far_kernel<<<grid_far, MF_THREADS, 0, st>>>(prep, n_lines, (const int2*)ranges, nu_min, step, n_nu, tile_samples,
-                                                   (int)chunks, cp, cutoff, l1_work, evals, work, tile_first);
+                                                   (int)chunks, cp, cutoff, l1_work, evals, work, tile_first, cg,
+                                                   (const int*)cells, cells + cell_head(cg));
   dim3 grid((unsigned)(n_tiles * chunks * parts), (unsigned)n_rows);
   // the staging buffers take the kernel past 48 KB of shared memory: opt in (per call, so
   // that every device and context the caller uses gets it; a host-side attribute write)

@@ -355,6 +355,7 @@ jac_far_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__ jpr
   const int tid = threadIdx.x, warp = tid >> 5;
   if ((tid & 31) == 0)
     for (int k = 0; k < MJ_NCOEF; ++k) s_part[warp][k] = 0.0;
+  __syncwarp();                                            // flush_nodes adds from other lanes
 
   float xa[MJ_K / 2], xb[MJ_KF / 2];
 #pragma unroll

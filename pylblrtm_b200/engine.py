@@ -702,11 +702,17 @@ class Job:
                   grid.n_nu, grid.tile_samples, self.cutoff, n_grp, od.data_ptr(), err.data_ptr(),
                   _lib.ptr(evals))
         if precision == "fp32":
-            l1_work = torch.empty((_lib.load().lbl_ml_work_floats(n_rows, grid.tile_samples, t_count),),
-                                  dtype=torch.float32, device=dev)
+            flags = _lib.LBL_DETERMINISTIC if deterministic else 0
+            n_l1 = -(-_lib.load().lbl_ml_work_floats(n_rows, grid.tile_samples, t_count) // 4) * 4
+            n_cells = _lib.load().lbl_line_cells_floats(n_rows, grid.n_nu, grid.tile_samples, grid.step, self.cutoff)
+            l1_work = torch.empty((n_l1 + n_cells,), dtype=torch.float32, device=dev)
+            if n_cells > 0:
+                flags |= _lib.LBL_LINE_CELLS
+                _lib.call("lbl_line_cells", d.lines, d.kept, prep.data_ptr(), n_kept, n_rows, grid.nu_min, grid.step,
+                          grid.n_nu, grid.tile_samples, self.cutoff, l1_work.data_ptr() + 4 * n_l1, stream)
+                self.launches += 2
             _lib.call("lbl_tau_tiles_ml_f32", common[0], common[1], common[2], d.inner, l1_work.data_ptr(),
-                      *common[3:], 0 if evals is None else evals.data_ptr() + 8, t_first, t_count,
-                      _lib.LBL_DETERMINISTIC if deterministic else 0, stream)
+                      *common[3:], 0 if evals is None else evals.data_ptr() + 8, t_first, t_count, flags, stream)
             self.launches += 1
         else:
             _lib.call("lbl_tau_tiles_f32" if single else "lbl_tau_tiles_f64", *common, stream)
