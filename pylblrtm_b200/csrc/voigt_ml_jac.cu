@@ -434,7 +434,9 @@ jac_ml_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__ jpre
     const int2 q = inner_ranges[tile];
     rng = make_int2(max(rng.x, q.x), min(rng.y, q.y));
   }
-  if (use_l1 && tid < MJ_NCOEF) s_c1[tid] = l1_coef[((long long)row * gridDim.x + blockIdx.x) * MJ_NCOEF + tid];
+  if (use_l1)                                       // CTAs of short tiles have fewer threads than coefficients
+    for (int i = tid; i < MJ_NCOEF; i += blockDim.x)
+      s_c1[i] = l1_coef[((long long)row * gridDim.x + blockIdx.x) * MJ_NCOEF + i];
   const int w0 = warp * MJ_WARP_PTS;
   const int n_w = max(0, min(MJ_WARP_PTS, n_c - w0));
   const float H2 = 0.5f * (float)(n_w - 1), C2w = (float)w0 + H2;

@@ -182,3 +182,19 @@ def test_jacobian_ranges_select_every_line(cuda, tile, monkeypatch):
     for a, b in zip(with_ranges, every):
         scale = b.abs().amax(dim=-1, keepdim=True).clamp_min(1e-30)
         assert ((a - b).abs() / scale).max().item() <= 5e-6
+
+
+@pytest.mark.parametrize("tile_pts", [70, 130, 250, 270])
+def test_jacobian_of_short_tiles(cuda, tile_pts):
+    """Tiles of 65 to 256 points run in CTAs of 32 or 64 threads, fewer than the level-1
+    coefficients: od and both derivatives against the same lines on long tiles' points, where
+    the windows admit the same lines (a cut-off that holds the whole list)."""
+    from pylblrtm_b200 import engine, synthetic
+    sd = synthetic.scale_strengths(synthetic.three_gas_lines(3000, 1498.0, 1506.0, seed=21), 1e-4)
+    li = engine.layer_input_from_profile(synthetic.logp_profile(4))
+    run = lambda pts: engine.Job(sd, li, engine.make_grid(1500.0, 1503.998, 0.002, (pts + 0.25) * 0.002), 40.0) \
+        .jacobian("H2O", deterministic=True)
+    for x, y in zip(run(tile_pts), run(1000)):
+        assert torch.isfinite(x).all()
+        scale = y.abs().amax(dim=2, keepdim=True)
+        assert ((x - y).abs() / scale).max().item() <= 5e-6      # two float32 splits of the same sums
