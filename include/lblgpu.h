@@ -240,6 +240,13 @@ long long lbl_line_cells_floats(int n_rows, long long n_nu, int tile_samples, do
 int lbl_line_cells(const LineIn* lines, const int* n_kept, const LineF32* prep, int n_lines, int n_rows, double nu_min,
                    double step, long long n_nu, int tile_samples, double cutoff, float* cells, void* stream);
 
+/* The same for lbl_jacobian_ml_f32 (three sums per cell): behind its level-1 coefficients, at
+ * l1_work + lbl_jacobian_ml_work_floats(...) rounded up to a multiple of 4. */
+long long lbl_line_cells_jac_floats(int n_rows, long long n_nu, int tile_samples, double step, double cutoff);
+int lbl_line_cells_jac(const LineIn* lines, const int* n_kept, const LineF32* prep, const LineJac* jprep, int n_lines,
+                       int n_rows, double nu_min, double step, long long n_nu, int tile_samples, double cutoff,
+                       float* cells, void* stream);
+
 /* Layer Jacobians by the multi-level float32 summation (no reference
  * counterpart; the retrieval adjoint): writes od (as lbl_tau_tiles_ml_f32),
  * d_t = d od / dT_layer and d_v = d od / d ln VMR_layer of the gas chosen in

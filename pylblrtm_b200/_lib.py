@@ -55,6 +55,8 @@ SIGNATURES = {
                                   _P]),
     "lbl_line_cells_floats": (_L, [_I, _L, _I, _D, _D]),
     "lbl_line_cells": (_I, [_P, _P, _P, _I, _I, _D, _D, _L, _I, _D, _P, _P]),
+    "lbl_line_cells_jac_floats": (_L, [_I, _L, _I, _D, _D]),
+    "lbl_line_cells_jac": (_I, [_P, _P, _P, _P, _I, _I, _D, _D, _L, _I, _D, _P, _P]),
     "lbl_ml_work_floats": (_L, [_I, _I, _I]),
     "lbl_line_prep_jac": (_I, [_P, _I, _P, _I, _I, _P, _P, _P, _P, _I, _P, _P, _P]),
     "lbl_jacobian_ml_f32": (_I, [_P, _P, _I, _P, _P, _P, _P, _I, _I, _D, _D, _L, _I, _D, _P, _P, _P, _P, _P, _P,

@@ -17,7 +17,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 PKG = os.path.dirname(HERE)
 ROOT = os.path.dirname(PKG)
 SOURCES = ["capi.cu", "prep.cu", "line_sort.cu", "voigt.cu", "voigt_f64.cu", "voigt_ml.cu", "voigt_ml_jac.cu", "mlp.cu"]
-HEADERS = ["lbl_common.cuh", "faddeeva.cuh", "sum_common.cuh", "weideman_coeffs.h", os.path.join("..", "..", "include", "lblgpu.h")]
+HEADERS = ["lbl_common.cuh", "line_cells.cuh", "cheb_tables.h", "faddeeva.cuh", "sum_common.cuh", "weideman_coeffs.h", os.path.join("..", "..", "include", "lblgpu.h")]
 LIB = os.path.join(PKG, "liblblgpu.so")
 HOST_LIB = os.path.join(PKG, "libfaddeeva_host.so")
 IO_LIB = os.path.join(PKG, "liblblio.so")

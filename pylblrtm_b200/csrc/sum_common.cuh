@@ -112,6 +112,22 @@ __device__ __forceinline__ LineJac line_jac_from_planes(const float4& p0, const 
   return J;
 }
 
+// Sum over the 32 lanes of f[16], transposed: afterwards lanes 2j and 2j+1 hold the
+// total of node j (j = (lane >> 1) & 15); 16 shuffles for the 16 sums.
+__device__ __forceinline__ float reduce_nodes16(const float (&f)[16], int lane) {
+  constexpr unsigned full = 0xffffffffu;
+  float g[8], h[4], u[2];
+  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4, b1 = lane & 2;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) g[k] = (b4 ? f[k + 8] : f[k]) + __shfl_xor_sync(full, b4 ? f[k] : f[k + 8], 16);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) h[k] = (b3 ? g[k + 4] : g[k]) + __shfl_xor_sync(full, b3 ? g[k] : g[k + 4], 8);
+#pragma unroll
+  for (int k = 0; k < 2; ++k) u[k] = (b2 ? h[k + 2] : h[k]) + __shfl_xor_sync(full, b2 ? h[k] : h[k + 2], 4);
+  const float v = (b1 ? u[1] : u[0]) + __shfl_xor_sync(full, b1 ? u[0] : u[1], 2);
+  return v + __shfl_xor_sync(full, v, 1);
+}
+
 // Adds the lanes' float node sums into the warp's float64 sums and clears them; every lane of
 // the warp calls it. K = 16 or 8. The sums are formed in float64 by a transposed reduction
 // (32 or 18 shuffles where a reduction per node took 160 or 80; the flush had been half of the

@@ -33,6 +33,7 @@
 #include "cheb_tables.h"
 #include "faddeeva.cuh"
 #include "lbl_common.cuh"
+#include "line_cells.cuh"
 #include "sum_common.cuh"
 
 namespace lbl {
@@ -149,52 +150,6 @@ __device__ __forceinline__ float clenshaw16(const float* c, float t) {
 // ~ 1e-8 of the cell's field; nothing cancels that the lines' own rounding would not show.
 constexpr int CELL_M = 11;                     // moments k = 1 .. 11
 constexpr int CELL_F = 16;                     // floats per record: moments, g_max, e_min, e_max, a_min, lines
-constexpr float CELL_RATIO = 1.0f / 6.5f;
-constexpr int CELL_MIN = 4;                    // fewer lines are cheaper one by one
-constexpr int CELL_MIN_CHUNKS = 16;            // fewer chunks on the grid: no cells
-constexpr int CELL_MIN_PTS = 64;               // smallest cell (bounds the records to 1 byte per point and row)
-
-struct CellGeom {
-  int wp, n;            // points per cell, cells (0: none)
-  long long off;        // cell q starts at grid index q * wp - off
-};
-
-// A quarter of a chunk per cell: far cells (beyond four half-widths) then have |zeta| / |D| of
-// about 1/13. No cells where no line can be that far, for chunks shorter than two cells, or
-// for a grid of few chunks (each cell serves them all). The rule looks at the grid alone, so
-// a shard or a batch of profiles takes the same cells as the full job.
-static CellGeom cell_geometry(long long n_nu, int tile_samples, double step, double cutoff) {
-  const long long nch = (tile_samples + ML_CHUNK - 1) / ML_CHUNK;
-  const long long n_c = tile_samples / nch;
-  CellGeom g = {0, 0, 0};
-  const double reach = cutoff / step;
-  if (n_c < 2 * CELL_MIN_PTS || !(reach > 2.0 * (double)n_c) || reach > 1.0e9 ||
-      (n_nu + tile_samples - 1) / tile_samples * nch < CELL_MIN_CHUNKS)
-    return g;
-  g.wp = (int)(n_c / 4 > CELL_MIN_PTS ? n_c / 4 : CELL_MIN_PTS);
-  g.off = ((long long)reach / g.wp + 2) * g.wp;
-  const long long n = (n_nu + 2 * g.off + g.wp - 1) / g.wp;
-  if (n > 0x3fffffff) return CellGeom{0, 0, 0};
-  g.n = (int)n;
-  return g;
-}
-
-// idx[q] = first sorted line whose unshifted centre is at or beyond the start of cell q (q <= n).
-__global__ void cell_bounds_kernel(const LineIn* __restrict__ lines, const int* __restrict__ n_kept, double nu_min,
-                                   double step, CellGeom cg, int* __restrict__ idx) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q > cg.n) return;
-  const double x = grid_nu(nu_min, step, (long long)q * cg.wp - cg.off);
-  int a = 0, b = *n_kept;
-  while (a < b) {
-    const int m = (a + b) >> 1;
-    if (lines[m].nu0 < x) a = m + 1; else b = m;
-  }
-  idx[q] = a;
-}
-
-__device__ __forceinline__ float reduce16_transposed(const float (&f)[ML_K], int lane);
-
 // One warp per (cell, row).
 __global__ void __launch_bounds__(256)
 line_moments_kernel(const LineF32* __restrict__ prep, int n_lines, const int* __restrict__ idx, CellGeom cg,
@@ -241,7 +196,7 @@ line_moments_kernel(const LineF32* __restrict__ prep, int n_lines, const int* __
       J = Jn;
     }
   }
-  const float v = reduce16_transposed(m, lane);        // lanes 2j, 2j + 1: moment j + 1
+  const float v = reduce_nodes16(m, lane);        // lanes 2j, 2j + 1: moment j + 1
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1) {
     e_min = fminf(e_min, __shfl_xor_sync(0xffffffffu, e_min, o));
@@ -277,7 +232,6 @@ constexpr int MF_THREADS = 64;                 // lines per round
 constexpr int MF_FLUSH = 32;                   // rounds summed in float before the double sums
 
 constexpr int MF_STAGES = 3;                   // rounds of line records in flight per thread
-constexpr int MF_CELLS = 512;                  // most cells of a tile's window (more: every line by itself)
 
 // amp * Re w by the far-wing form (amp_far = amp y / sqrt(pi)), added to f (|z|^2 >= FAR_Z2, y >= 0).
 __device__ __forceinline__ void far_wing_add(float& f, float x, float y2, float ny2, float amp_far) {
@@ -326,9 +280,7 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
   __shared__ double s_part[MF_THREADS / 32][ML_K + ML_KF];
   __shared__ float s_coef[ML_K + ML_KF];
   __shared__ unsigned s_cnt[3];
-  __shared__ int s_use[MF_CELLS];                          // cells evaluated through their moments
-  __shared__ int s_dir[MF_CELLS], s_pre[MF_CELLS + 1];     // stretches of other lines: start, lines before
-  __shared__ int s_wu[MF_THREADS / 32], s_wd[MF_THREADS / 32], s_wl[MF_THREADS / 32];   // per-warp scan totals
+  __shared__ LineSplit<MF_THREADS> s_split;
   __shared__ float s_cell[MF_THREADS / 32][ML_KF];
 
   const int row = blockIdx.y;
@@ -364,92 +316,22 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
 
   // ---- the tile's lines split into cells to evaluate by their moments and other lines
   int n_use = 0, n_dir = 1, n_direct = max(0, rng.y - rng.x);
-  if (cg.n > 0 && n_direct > 0) {
-    // the window in cells, with two cells on either side for shifted lines (checked below)
-    const double win0 = cutoff / step;
-    const int qa = (int)max(0LL, (t0 - (long long)win0 + cg.off) / cg.wp - 3);
-    const int qe = (int)min((long long)cg.n, (t1 + (long long)win0 + cg.off) / cg.wp + 3);
-    if (qe - qa <= MF_CELLS && cell_idx[qa] <= rng.x && cell_idx[qe] >= rng.y) {
-      const float* rr = cell_rec + (long long)row * cg.n * CELL_F;
-      const double wl = (double)(t0 - c0) - win0 + 1.0, wr = (double)(t1 - 1 - c0) + win0 - 1.0;   // a point of margin
-      const float half = 0.5f * (float)cg.wp;
-      n_dir = 0;
-      n_direct = 0;
-      for (int q0 = qa; q0 < qe; q0 += MF_THREADS) {
-        const int q = q0 + tid;
-        int i0 = 0, len = 0;
-        bool use = false;
-        if (q < qe) {
-          const int a = cell_idx[q], b = cell_idx[q + 1];
-          i0 = max(a, rng.x);
-          len = max(0, min(b, rng.y) - i0);
-          if (len > 0) {
-            const float4 m = *reinterpret_cast<const float4*>(rr + (long long)q * CELL_F + CELL_F - 4);
-            const float g_max = rr[(long long)q * CELL_F + CELL_M];
-            if (m.w == 0.f) len = 0;                       // only inactive lines
-            const float pc = (float)((long long)q * cg.wp - cg.off - c0) + half;
-            const float lo = pc + m.x, hi = pc + m.y;
-            // all lines beyond four half-widths on one side, inside the window, in the far-wing
-            // regime at the nearest node and well inside the series' radius
-            const float gap = fmaxf(lo - (C1 + H1), (C1 - H1) - hi);
-            const float z = fmaxf(fabsf(m.x), fabsf(m.y)) + g_max, D = fabsf(pc - C1) - H1;
-            use = m.w >= (float)CELL_MIN && i0 == a && len == b - a && gap > ML_FAR1 * H1 + 2.f && (double)lo >= wl &&
-                  (double)hi <= wr && m.z * gap >= 50.f && z <= CELL_RATIO * D;
-          }
-        }
-        const unsigned bu = __ballot_sync(0xffffffffu, use), bd = __ballot_sync(0xffffffffu, len > 0 && !use);
-        int pl = len > 0 && !use ? len : 0;                // inclusive scan of the other lines
-        const int own = pl;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int u = __shfl_up_sync(0xffffffffu, pl, o);
-          if (lane >= o) pl += u;
-        }
-        if (lane == 31) {
-          s_wu[warp] = __popc(bu);
-          s_wd[warp] = __popc(bd);
-          s_wl[warp] = pl;
-        }
-        __syncthreads();
-        int ou = n_use, od = n_dir, ol = n_direct;
-        for (int w = 0; w < MF_THREADS / 32; ++w) {
-          if (w < warp) {
-            ou += s_wu[w];
-            od += s_wd[w];
-            ol += s_wl[w];
-          }
-          n_use += s_wu[w];
-          n_dir += s_wd[w];
-          n_direct += s_wl[w];
-        }
-        const unsigned lt = (1u << lane) - 1u;
-        if (use) s_use[ou + __popc(bu & lt)] = q;
-        if (own > 0) {
-          const int o = od + __popc(bd & lt);
-          s_dir[o] = i0;
-          s_pre[o] = ol + pl - own;
-        }
-        __syncthreads();
-      }
-      if (tid == 0) s_pre[n_dir] = n_direct;
-    }
-  }
+  const float* const rec_row = cell_rec + (long long)row * cg.n * CELL_F;
+  const bool split = split_lines<MF_THREADS, CELL_F, CELL_M>(s_split, cg, cell_idx, rec_row, rng, t0, t1, c0, H1,
+                                                             cutoff, step, n_use, n_dir, n_direct);
   const bool cells = n_use > 0;
-  const bool split = cg.n > 0 && !(n_dir == 1 && n_direct == rng.y - rng.x && !cells);
-  __syncthreads();
   if (cells) {                                             // thread: node tid % 8 of cells tid / 8, + 32, ...
     const int k = tid & (ML_KF - 1);
     const float xk = k < ML_KF / 2 ? H1 * c_node8[k] : -H1 * c_node8[ML_KF - 1 - k];
-    const float* rr = cell_rec + (long long)row * cg.n * CELL_F;
     const float half = 0.5f * (float)cg.wp;
     float f = 0.f;
     unsigned c = 0;
 #pragma unroll 4
     for (int i = tid >> 3; i < n_use; i += MF_THREADS / 8) {
-      const int q = s_use[i];
-      const float4* r4 = reinterpret_cast<const float4*>(rr + (long long)q * CELL_F);
+      const int q = s_split.use[i];
+      const float4* r4 = reinterpret_cast<const float4*>(rec_row + (long long)q * CELL_F);
       const float4 a = r4[0], b = r4[1], d = r4[2];
-      if (k == 0) c += (unsigned)rr[(long long)q * CELL_F + CELL_F - 1];
+      if (k == 0) c += (unsigned)rec_row[(long long)q * CELL_F + CELL_F - 1];
       const float D = (C1 + xk) - ((float)((long long)q * cg.wp - cg.off - c0) + half);
       const float rD = 1.0f / D, t = half * rD;
       float v = fmaf(d.z, t, d.y);
@@ -478,15 +360,7 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
   auto issue = [&](int r, int stage) {
     const int slot = r * MF_THREADS + tid;
     if (slot < n_direct) {   // prep records: 32 B each in a 256-B aligned allocation
-      int li = rng.x + slot;
-      if (split) {           // the stretch that holds this slot
-        int a = 0, b = n_dir - 1;
-        while (a < b) {
-          const int m = (a + b + 1) >> 1;
-          if (s_pre[m] <= slot) a = m; else b = m - 1;
-        }
-        li = s_dir[a] + (slot - s_pre[a]);
-      }
+      const int li = split ? split_line(s_split, n_dir, slot) : rng.x + slot;
       const float4* g = reinterpret_cast<const float4*>(lp + li);
       float4* d = reinterpret_cast<float4*>(&s_line[stage][tid]);
       cp_async16(d, g);
@@ -590,22 +464,7 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
 constexpr int ML_NBW = 128;                    // near items buffered per warp (bit-reproducible mode)
 constexpr unsigned FULL_MASK = 0xffffffffu;
 
-// Sum over the 32 lanes of f[16], transposed: afterwards lanes 2j and 2j+1 hold the
-// total of node j (j = (lane >> 1) & 15); 16 shuffles for the 16 sums.
-__device__ __forceinline__ float reduce16_transposed(const float (&f)[ML_K], int lane) {
-  float g[8], h[4], u[2];
-  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4, b1 = lane & 2;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) g[k] = (b4 ? f[k + 8] : f[k]) + __shfl_xor_sync(FULL_MASK, b4 ? f[k] : f[k + 8], 16);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) h[k] = (b3 ? g[k + 4] : g[k]) + __shfl_xor_sync(FULL_MASK, b3 ? g[k] : g[k + 4], 8);
-#pragma unroll
-  for (int k = 0; k < 2; ++k) u[k] = (b2 ? h[k + 2] : h[k]) + __shfl_xor_sync(FULL_MASK, b2 ? h[k] : h[k + 2], 4);
-  float v = (b1 ? u[1] : u[0]) + __shfl_xor_sync(FULL_MASK, b1 ? u[0] : u[1], 2);
-  return v + __shfl_xor_sync(FULL_MASK, v, 1);
-}
-
-// The same for f[8]: afterwards lanes 4j .. 4j+3 hold the total of node j = (lane >> 2) & 7.
+// reduce_nodes16 for f[8]: afterwards lanes 4j .. 4j+3 hold the total of node j = (lane >> 2) & 7.
 __device__ __forceinline__ float reduce8_transposed(const float (&f)[ML_KF], int lane) {
   float g[4], h[2];
   const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
@@ -899,7 +758,7 @@ tau_ml_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restr
 #pragma unroll
       for (int k = 0; k < ML_K; ++k) f[k] = 0.f;
       level2_lines<ML_K>(f, s_l2[warp], 1, n2w, s_g, s_h, s_p, s_q, C2w, H2, lane);
-      const float v = reduce16_transposed(f, lane);
+      const float v = reduce_nodes16(f, lane);
       if (!(lane & 1)) s_n2[warp][(lane >> 1) & 15] += (double)v;
     }
     if (n2fw > 0) {
@@ -1153,12 +1012,9 @@ extern "C" long long lbl_ml_work_floats(int n_rows, int tile_samples, int tile_c
   return (long long)n_rows * tile_count * chunks * (ML_K + ML_KF);
 }
 
-// Layout of the line cells: cell bounds (int, n + 1, padded to 4), then the records.
-static long long cell_head(const CellGeom& g) { return ((long long)g.n + 1 + 3) / 4 * 4; }
-
 extern "C" long long lbl_line_cells_floats(int n_rows, long long n_nu, int tile_samples, double step, double cutoff) {
   if (n_rows < 1 || n_nu < 1 || tile_samples < 1 || !(step > 0) || !(cutoff >= 0)) return -1;
-  const CellGeom g = cell_geometry(n_nu, tile_samples, step, cutoff);
+  const CellGeom g = cell_geometry(n_nu, tile_samples, step, cutoff, ML_CHUNK);
   return g.n == 0 ? 0 : cell_head(g) + (long long)n_rows * g.n * CELL_F;
 }
 
@@ -1168,7 +1024,7 @@ extern "C" int lbl_line_cells(const LineIn* lines, const int* n_kept, const Line
   if (!lines || !n_kept || !prep || !cells || n_lines < 1 || n_rows < 1 || n_rows > 65535 || n_nu < 1 ||
       tile_samples < 1 || !(step > 0) || !(cutoff >= 0) || ((uintptr_t)cells) % 16)
     return lbl_set_error(LBL_EINVAL, "lbl_line_cells: bad arguments");
-  const CellGeom g = cell_geometry(n_nu, tile_samples, step, cutoff);
+  const CellGeom g = cell_geometry(n_nu, tile_samples, step, cutoff, ML_CHUNK);
   if (g.n == 0) return LBL_OK;
   const cudaStream_t st = (cudaStream_t)stream;
   cell_bounds_kernel<<<g.n / 128 + 1, 128, 0, st>>>(lines, n_kept, nu_min, step, g, (int*)cells);
@@ -1204,7 +1060,7 @@ extern "C" int lbl_tau_tiles_ml_f32(const LineF32* prep, int n_lines, const int*
   CellGeom cg = {0, 0, 0};
   const float* cells = nullptr;
   if (flags & LBL_LINE_CELLS) {
-    cg = cell_geometry(n_nu, tile_samples, step, cutoff);
+    cg = cell_geometry(n_nu, tile_samples, step, cutoff, ML_CHUNK);
     cells = l1_work + ((long long)n_rows * n_tiles * chunks * (ML_K + ML_KF) + 3) / 4 * 4;
     if (((uintptr_t)l1_work) % 16)
       return lbl_set_error(LBL_EINVAL, "lbl_tau_tiles_ml_f32: l1_work must be 16-byte aligned");

@@ -25,6 +25,7 @@
 #include "cheb_tables.h"
 #include "faddeeva.cuh"
 #include "lbl_common.cuh"
+#include "line_cells.cuh"
 #include "sum_common.cuh"
 
 namespace lbl {
@@ -44,7 +45,12 @@ static __constant__ double c_jdct16[MJ_K * MJ_K] = {LBL_DCT16};
 constexpr int MJ_KF = 8;                           // nodes for level-1 lines beyond four half-widths
 constexpr float MJ_FAR1 = 3.f;                     // "far": more than (1 + MJ_FAR1) half-widths from the centre
 constexpr int MJ_NCOEF = 3 * (MJ_K + MJ_KF);       // level-1 coefficients per (chunk, row)
-constexpr int MJF_THREADS = 256;                   // lines per round of jac_far_kernel
+// Level 1 is latency-bound once its far lines come as cells: small CTAs cover each other's
+// waits. 200 cm^-1, 60 layers, 26,000 lines on B200: every line by itself 1,235 us (1,100 with
+// the transposed flush); with cells and CTAs of 256, 128 and 64 threads 551, 393 and 337 us
+// (plus 66 us for the moments); 6 instead of 8 CTAs per SM 385 us.
+constexpr int MJF_THREADS = 64;                    // lines per round of jac_far_kernel
+constexpr int MJF_CTAS = 8;                        // per SM
 constexpr int MJF_STAGES = 2;                      // rounds of line records in flight per thread
 constexpr int MJF_FLUSH = 32;                      // rounds summed in float before the double sums
 static __constant__ float c_jnode8[MJ_KF] = {LBL_CHEB8_NODES};
@@ -266,13 +272,103 @@ __device__ __forceinline__ void jfar_line(float (&f)[3][K], const float (&xs)[K 
   }
 }
 
+// Line cells of the three sums (line_cells.cuh; the expansion of voigt_ml.cu). With v = 1/(delta -
+// ig), delta and g in points, the two leading terms of w and w' give, times sqrt(pi),
+//   u     = Im v / a + Im v^3 / (2 a^3)
+//   -x u_x = (Im v + g Re v^2) / a + 3 (Im v^3 + g Re v^4) / (2 a^3)
+//   u_y   = Re v^2 / a^2 + 3 Re v^4 / (2 a^4),  -u_x = Im v^2 / a^2 + 3 Im v^4 / (2 a^4)
+// and v^n = sum_k C(k, n-1) zeta^(k-n+1) / D^(k+1), so each weighted sum is again a series in
+// 1/D with real moments. Three times eleven moments per (cell, row).
+constexpr int JC_M = 11;                           // moments per sum
+constexpr int JC_F = 40;                           // floats per record: 3 x (11 + 1), extent and count
+constexpr int JC_G = JC_M;                         // slot of g_max (the first sum's spare)
+
+__global__ void __launch_bounds__(256)
+jac_moments_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__ jprep, int n_lines,
+                   const int* __restrict__ idx, CellGeom cg, float* __restrict__ rec) {
+  const int q = blockIdx.x * 8 + (threadIdx.x >> 5), row = blockIdx.y, lane = threadIdx.x & 31;
+  if (q >= cg.n) return;
+  float* out = rec + ((long long)row * cg.n + q) * JC_F;
+  const int i0 = idx[q], i1 = idx[q + 1];
+  if (i1 <= i0) {                                  // empty: only the count is read
+    if (lane == 0) out[JC_F - 1] = 0.f;
+    return;
+  }
+  const LineF32* lp = prep + (long long)row * n_lines;
+  const LineJac* jp = jprep + (long long)row * n_lines;
+  const int jb = (int)((long long)q * cg.wp - cg.off);
+  const float s = 0.5f * (float)cg.wp, inv_s = 1.0f / s;
+  float m[3][MJ_K];
+#pragma unroll
+  for (int p = 0; p < 3; ++p)
+#pragma unroll
+    for (int k = 0; k < MJ_K; ++k) m[p][k] = 0.f;
+  float e_min = 3.0e38f, e_max = -3.0e38f, a_min = 3.0e38f, g_max = 0.f;
+  int cnt = 0;
+  bool ok = true;
+  for (int li = i0 + lane; li < i1; li += 32) {
+    const LineF32 L = lp[li];
+    if (!(L.nuc == L.nuc)) continue;               // inactive
+    const LineJac J = jp[li];
+    ++cnt;
+    const float ia = 1.0f / L.a;
+    const float e = (float)(L.j0 - jb) - s + L.b * ia, g = L.y * ia;
+    ok = ok && L.y >= 0.f && L.a > 0.f && g <= s;  // broad lines (or a negative width): line by line
+    e_min = fminf(e_min, e);
+    e_max = fmaxf(e_max, e);
+    a_min = fminf(a_min, L.a);
+    g_max = fmaxf(g_max, g);
+    const float zr = e * inv_s, zi = g * inv_s, k0 = float(INV_SQRT_PI);
+    const float w0 = k0 * L.amp, wu = k0 * J.jT_u, wx = k0 * J.jT_x, wy = k0 * J.jT_y;
+    const float vu = k0 * J.jv_u, vy = k0 * J.jv_y, vx = k0 * J.jv_x;
+    const float ia2 = ia * ia, c3 = inv_s * ia2, c4 = inv_s * inv_s * ia2;   // 1/(s a^2), 1/(s^2 a^2)
+    // R, I: real and imaginary part of (zeta / s)^k; R1.. one, two and three powers before
+    float R = zr, I = zi, R1 = 1.f, I1 = 0.f, R2 = 0.f, I2 = 0.f, R3 = 0.f, I3 = 0.f;
+#pragma unroll
+    for (int k = 1; k <= JC_M; ++k) {
+      const float c2k = 0.5f * (float)(k * (k - 1)), c3k = (float)(k * (k - 1) * (k - 2)) / 6.0f;
+      const float iv = s * I, rv2 = (float)k * R1, iv2 = (float)k * I1;
+      const float iv3 = c2k * c3 * I2, rv4 = c3k * c4 * R3, iv4 = c3k * c4 * I3;   // over a^2
+      const float U = ia * fmaf(0.5f, iv3, iv);
+      const float X = ia * fmaf(1.5f, fmaf(g, rv4, iv3), fmaf(g, rv2, iv));
+      const float Y = ia2 * fmaf(1.5f, rv4, rv2), Z = ia2 * fmaf(1.5f, iv4, iv2);
+      m[0][k - 1] = fmaf(w0, U, m[0][k - 1]);
+      m[1][k - 1] = fmaf(wu, U, fmaf(wx, X, fmaf(-wy, Y, m[1][k - 1])));
+      m[2][k - 1] = fmaf(vu, U, fmaf(vy, Y, fmaf(vx, Z, m[2][k - 1])));
+      const float Rn = fmaf(R, zr, -I * zi), In = fmaf(R, zi, I * zr);
+      R3 = R2; I3 = I2; R2 = R1; I2 = I1; R1 = R; I1 = I; R = Rn; I = In;
+    }
+  }
+#pragma unroll
+  for (int p = 0; p < 3; ++p) {
+    const float v = reduce_nodes16(m[p], lane);    // lanes 2j, 2j + 1: moment j + 1
+    if (!(lane & 1) && (lane >> 1) < JC_M) out[p * (JC_M + 1) + (lane >> 1)] = v;
+  }
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    e_min = fminf(e_min, __shfl_xor_sync(0xffffffffu, e_min, o));
+    e_max = fmaxf(e_max, __shfl_xor_sync(0xffffffffu, e_max, o));
+    a_min = fminf(a_min, __shfl_xor_sync(0xffffffffu, a_min, o));
+    g_max = fmaxf(g_max, __shfl_xor_sync(0xffffffffu, g_max, o));
+  }
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  ok = __all_sync(0xffffffffu, ok);
+  if (lane == 1) {
+    out[JC_G] = g_max;
+    out[JC_F - 4] = e_min;
+    out[JC_F - 3] = e_max;
+    out[JC_F - 2] = a_min;
+    out[JC_F - 1] = ok ? (float)cnt : -1.f;
+  }
+}
+
 // One pass of jac_far_kernel over the tile's candidate lines for the lines of one node
 // class (K = MJ_K: level-1 lines within four half-widths; K = MJ_KF: beyond); the warp's
 // float64 sums of that class go to row[q * K + k]. Two passes keep 3 K accumulators live
 // instead of 3 (MJ_K + MJ_KF).
-template <int K>
+template <int K, typename LineOf>
 __device__ __forceinline__ void jfar_pass(float4 (*s_line)[4][MJF_THREADS], const LineF32* lp, const LineJac* jp,
-                                          int2 rng, double wlo, double whi, long long c0, float H1,
+                                          int n, LineOf line_of, double wlo, double whi, long long c0, float H1,
                                           const float (&xs)[K / 2], double* row) {
   const int tid = threadIdx.x, lane = tid & 31;
   const float C1 = H1;
@@ -281,12 +377,13 @@ __device__ __forceinline__ void jfar_pass(float4 (*s_line)[4][MJF_THREADS], cons
   for (int q = 0; q < 3; ++q)
 #pragma unroll
     for (int k = 0; k < K; ++k) f[q][k] = 0.f;
-  // records of round r (line rng.x + r * MJF_THREADS + tid) go to stage r % 2, one round
-  // ahead; each thread copies into and reads only its own slots
-  const int n_rounds = rng.y > rng.x ? (rng.y - rng.x + MJF_THREADS - 1) / MJF_THREADS : 0;
+  // records of round r (line line_of(r * MJF_THREADS + tid) of the pass's n) go to stage r % 2,
+  // one round ahead; each thread copies into and reads only its own slots
+  const int n_rounds = (n + MJF_THREADS - 1) / MJF_THREADS;
   auto issue = [&](int r, int stage) {
-    const int li = rng.x + r * MJF_THREADS + tid;
-    if (li < rng.y) {   // 32-B records in 256-B aligned allocations
+    const int slot = r * MJF_THREADS + tid;
+    if (slot < n) {     // 32-B records in 256-B aligned allocations
+      const int li = line_of(slot);
       const float4* g = reinterpret_cast<const float4*>(lp + li);
       const float4* h = reinterpret_cast<const float4*>(jp + li);
       cp_async16(&s_line[stage][0][tid], g);
@@ -302,7 +399,7 @@ __device__ __forceinline__ void jfar_pass(float4 (*s_line)[4][MJF_THREADS], cons
     const int stage = r & 1;
     issue(r + 1, stage ^ 1);                                // the stage read last round
     cp_async_wait<1>();
-    const bool have = rng.x + r * MJF_THREADS + tid < rng.y;
+    const bool have = r * MJF_THREADS + tid < n;
     JFarLine R;
     if (have) {
       R.l = line_f32_from_planes(s_line[stage][0][tid], s_line[stage][1][tid]);
@@ -330,11 +427,14 @@ __device__ __forceinline__ void jfar_pass(float4 (*s_line)[4][MJF_THREADS], cons
   for (int q = 0; q < 3; ++q) flush_nodes(f[q], row + q * K, lane);
 }
 
-__global__ void __launch_bounds__(MJF_THREADS, 2)
+__global__ void __launch_bounds__(MJF_THREADS, MJF_CTAS)
 jac_far_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__ jprep, int n_lines,
                const int2* __restrict__ ranges, const int2* __restrict__ near_ranges, double nu_min, double step,
                long long n_nu, int tile_samples, int chunks_per_tile, int chunk_pts, double cutoff,
-               float* __restrict__ l1_coef) {
+               float* __restrict__ l1_coef, CellGeom cg, const int* __restrict__ cell_idx,
+               const float* __restrict__ cell_rec) {
+  __shared__ LineSplit<MJF_THREADS> s_split;
+  __shared__ float s_cell[MJF_THREADS / 32][3][MJ_KF];
   __shared__ __align__(16) float4 s_line[MJF_STAGES][4][MJF_THREADS];  // 64-B records as four 16-B planes
   __shared__ double s_part[MJF_THREADS / 32][MJ_NCOEF];                 // [q][16] then [q][8] per warp
 
@@ -369,27 +469,73 @@ jac_far_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__ jpr
     const int2 q = near_ranges[tile];
     rng16 = make_int2(max(rng.x, q.x), min(rng.y, q.y));
   }
-  jfar_pass<MJ_K>(s_line, lp, jp, rng16, wlo, whi, c0, H1, xa, s_part[warp]);
-  jfar_pass<MJ_KF>(s_line, lp, jp, rng, wlo, whi, c0, H1, xb, s_part[warp] + 3 * MJ_K);
+  jfar_pass<MJ_K>(s_line, lp, jp, max(0, rng16.y - rng16.x), [&](int i) { return rng16.x + i; }, wlo, whi, c0, H1, xa,
+                  s_part[warp]);
+  // beyond four half-widths: cells by their moments, one thread per (cell, node), and the
+  // lines of the other cells one by one
+  int n_use = 0, n_dir = 1, n_direct = max(0, rng.y - rng.x);
+  const float* const rec_row = cell_rec + (long long)row * cg.n * JC_F;
+  const bool split = split_lines<MJF_THREADS, JC_F, JC_G>(s_split, cg, cell_idx, rec_row, rng, t0, t1, c0, H1, cutoff,
+                                                          step, n_use, n_dir, n_direct);
+  if (n_use > 0) {
+    const int k = tid & (MJ_KF - 1);
+    const float xk = k < MJ_KF / 2 ? H1 * c_jnode8[k] : -H1 * c_jnode8[MJ_KF - 1 - k];
+    const float half = 0.5f * (float)cg.wp;
+    float f[3] = {0.f, 0.f, 0.f};
+    for (int i = tid >> 3; i < n_use; i += MJF_THREADS / 8) {
+      const int q = s_split.use[i];
+      const float4* r4 = reinterpret_cast<const float4*>(rec_row + (long long)q * JC_F);
+      const float D = (H1 + xk) - ((float)((long long)q * cg.wp - cg.off - c0) + half);
+      const float rD = 1.0f / D, t = half * rD;
+      float4 c[9];
+#pragma unroll
+      for (int p = 0; p < 9; ++p) c[p] = r4[p];
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        const float4 a = c[3 * p], b = c[3 * p + 1], d = c[3 * p + 2];
+        float v = fmaf(d.z, t, d.y);
+        v = fmaf(v, t, d.x);
+        v = fmaf(v, t, b.w);
+        v = fmaf(v, t, b.z);
+        v = fmaf(v, t, b.y);
+        v = fmaf(v, t, b.x);
+        v = fmaf(v, t, a.w);
+        v = fmaf(v, t, a.z);
+        v = fmaf(v, t, a.y);
+        v = fmaf(v, t, a.x);
+        f[p] = fmaf(rD * rD, v, f[p]);
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      f[p] += __shfl_xor_sync(0xffffffffu, f[p], 8);
+      f[p] += __shfl_xor_sync(0xffffffffu, f[p], 16);
+      if ((tid & 31) < MJ_KF) s_cell[warp][p][tid & 31] = f[p];
+    }
+  }
+  jfar_pass<MJ_KF>(s_line, lp, jp, n_direct, [&](int i) { return split ? split_line(s_split, n_dir, i) : rng.x + i; },
+                   wlo, whi, c0, H1, xb, s_part[warp] + 3 * MJ_K);
   __syncthreads();
-  if (tid < MJ_NCOEF) {                                    // column tid: only this thread touches it
+  for (int c = tid; c < MJ_NCOEF; c += MJF_THREADS) {      // column c: only this thread touches it
     double v = 0.0;
-    for (int w = 0; w < MJF_THREADS / 32; ++w) v += s_part[w][tid];
-    s_part[0][tid] = v;
+    for (int w = 0; w < MJF_THREADS / 32; ++w) v += s_part[w][c];
+    if (n_use > 0 && c >= 3 * MJ_K)
+      for (int w = 0; w < MJF_THREADS / 32; ++w) v += (double)(&s_cell[w][0][0])[c - 3 * MJ_K];
+    s_part[0][c] = v;
   }
   __syncthreads();
-  if (tid < MJ_NCOEF) {                                    // Chebyshev coefficients (DCT)
+  for (int tc = tid; tc < MJ_NCOEF; tc += MJF_THREADS) {   // Chebyshev coefficients (DCT)
     double c = 0.0;
-    if (tid < 3 * MJ_K) {
-      const int q = tid / MJ_K, k = tid % MJ_K;
+    if (tc < 3 * MJ_K) {
+      const int q = tc / MJ_K, k = tc % MJ_K;
       for (int j = 0; j < MJ_K; ++j) c += s_part[0][q * MJ_K + j] * c_jdct16[k * MJ_K + j];
       c *= 2.0 / MJ_K;
     } else {
-      const int q = (tid - 3 * MJ_K) / MJ_KF, k = (tid - 3 * MJ_K) % MJ_KF;
+      const int q = (tc - 3 * MJ_K) / MJ_KF, k = (tc - 3 * MJ_K) % MJ_KF;
       for (int j = 0; j < MJ_KF; ++j) c += s_part[0][3 * MJ_K + q * MJ_KF + j] * c_jdct8[k * MJ_KF + j];
       c *= 2.0 / MJ_KF;
     }
-    l1_coef[((long long)row * gridDim.x + blockIdx.x) * MJ_NCOEF + tid] = (float)c;
+    l1_coef[((long long)row * gridDim.x + blockIdx.x) * MJ_NCOEF + tc] = (float)c;
   }
 }
 
@@ -869,6 +1015,28 @@ extern "C" int lbl_jac_near_ranges(const LineIn* lines, const int* n_kept, doubl
                          n_tiles, near, stream);
 }
 
+extern "C" long long lbl_line_cells_jac_floats(int n_rows, long long n_nu, int tile_samples, double step,
+                                               double cutoff) {
+  if (n_rows < 1 || n_nu < 1 || tile_samples < 1 || !(step > 0) || !(cutoff >= 0)) return -1;
+  const CellGeom g = cell_geometry(n_nu, tile_samples, step, cutoff, MJ_CHUNK);
+  return g.n == 0 ? 0 : cell_head(g) + (long long)n_rows * g.n * JC_F;
+}
+
+extern "C" int lbl_line_cells_jac(const LineIn* lines, const int* n_kept, const LineF32* prep, const LineJac* jprep,
+                                  int n_lines, int n_rows, double nu_min, double step, long long n_nu, int tile_samples,
+                                  double cutoff, float* cells, void* stream) {
+  if (!lines || !n_kept || !prep || !jprep || !cells || n_lines < 1 || n_rows < 1 || n_rows > 65535 || n_nu < 1 ||
+      tile_samples < 1 || !(step > 0) || !(cutoff >= 0) || ((uintptr_t)cells) % 16)
+    return lbl_set_error(LBL_EINVAL, "lbl_line_cells_jac: bad arguments");
+  const CellGeom g = cell_geometry(n_nu, tile_samples, step, cutoff, MJ_CHUNK);
+  if (g.n == 0) return LBL_OK;
+  const cudaStream_t st = (cudaStream_t)stream;
+  cell_bounds_kernel<<<g.n / 128 + 1, 128, 0, st>>>(lines, n_kept, nu_min, step, g, (int*)cells);
+  dim3 grid((unsigned)((g.n + 7) / 8), (unsigned)n_rows);
+  jac_moments_kernel<<<grid, 256, 0, st>>>(prep, jprep, n_lines, (const int*)cells, g, cells + cell_head(g));
+  return lbl_check_launch("lbl_line_cells_jac");
+}
+
 extern "C" int lbl_jacobian_ml_f32(const LineF32* prep, const LineJac* jprep, int n_lines, const int* ranges,
                                    const int* inner, const int* near, const double* t_layer, int n_rows, int n_lay, double nu_min,
                                    double step, long long n_nu, int tile_samples, double cutoff, float* l1_work,
@@ -885,8 +1053,18 @@ extern "C" int lbl_jacobian_ml_f32(const LineF32* prep, const LineJac* jprep, in
   if (n_tiles * chunks > 0x7fffffffLL) return lbl_set_error(LBL_EINVAL, "lbl_jacobian_ml_f32: grid too large");
   dim3 grid((unsigned)(n_tiles * chunks), (unsigned)n_rows);
   cudaStream_t st = (cudaStream_t)stream;
+  // with LBL_LINE_CELLS the line cells follow the level-1 coefficients (16-byte aligned)
+  CellGeom cg = {0, 0, 0};
+  const float* cells = nullptr;
+  if (flags & LBL_LINE_CELLS) {
+    cg = cell_geometry(n_nu, tile_samples, step, cutoff, MJ_CHUNK);
+    cells = l1_work + ((long long)n_rows * n_tiles * chunks * MJ_NCOEF + 3) / 4 * 4;
+    if (((uintptr_t)l1_work) % 16)
+      return lbl_set_error(LBL_EINVAL, "lbl_jacobian_ml_f32: l1_work must be 16-byte aligned");
+  }
   jac_far_kernel<<<grid, MJF_THREADS, 0, st>>>(prep, jprep, n_lines, (const int2*)ranges, (const int2*)near, nu_min,
-                                               step, n_nu, tile_samples, (int)chunks, cp, cutoff, l1_work);
+                                               step, n_nu, tile_samples, (int)chunks, cp, cutoff, l1_work, cg,
+                                               (const int*)cells, cells + cell_head(cg));
   if (flags & LBL_DETERMINISTIC) {
     constexpr int dyn_bytes = (MJ_THREADS / 32) * 3 * MJ_NBW * (int)sizeof(float);   // near-item buffers
     int dev = 0;

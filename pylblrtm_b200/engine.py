@@ -772,8 +772,14 @@ def _jacobian_impl(job: Job, gas: str, g_tau=None, deterministic: bool = False):
               stream)
     job.launches += 3                       # line prep and the two kernels of the Jacobian's
     flags = _lib.LBL_DETERMINISTIC if deterministic else 0
-    l1_work = torch.empty((_lib.load().lbl_jacobian_ml_work_floats(n_rows, n_nu, grid.tile_samples),),
-                          dtype=torch.float32, device=dev)
+    n_l1 = -(-_lib.load().lbl_jacobian_ml_work_floats(n_rows, n_nu, grid.tile_samples) // 4) * 4
+    n_cells = _lib.load().lbl_line_cells_jac_floats(n_rows, n_nu, grid.tile_samples, grid.step, job.cutoff)
+    l1_work = torch.empty((n_l1 + n_cells,), dtype=torch.float32, device=dev)
+    if n_cells > 0:
+        flags |= _lib.LBL_LINE_CELLS
+        _lib.call("lbl_line_cells_jac", d.lines, d.kept, prep.data_ptr(), jprep.data_ptr(), n_kept, n_rows,
+                  grid.nu_min, grid.step, n_nu, grid.tile_samples, job.cutoff, l1_work.data_ptr() + 4 * n_l1, stream)
+        job.launches += 2
     job.launches += 2                       # the two Jacobian kernels
     common = (prep.data_ptr(), jprep.data_ptr(), n_kept, d.ranges, d.inner, d.near, d.t_layer, n_rows, n_lay, grid.nu_min, grid.step, n_nu, grid.tile_samples, job.cutoff,
               l1_work.data_ptr())

@@ -68,6 +68,36 @@ def test_cells_against_lines_and_float64(cuda, case, monkeypatch):
     assert l2(with_cells.od) <= 1.2 * l2(by_line.od) + 2e-8
 
 
+@pytest.mark.parametrize("case", [c for c in CASES if c[0] != 60_000 or c[5] == 6])
+def test_jacobian_cells_against_lines(cuda, case, monkeypatch):
+    """The three Jacobian sums and the vector-Jacobian product with and without cells."""
+    job = _job(*case, seed=int(case[0]) + 1)
+    grid = job.grid
+    assert _lib.load().lbl_line_cells_jac_floats(1, grid.n_nu, grid.tile_samples, grid.step, job.cutoff) > 0
+    g = torch.rand((1, grid.n_nu), generator=torch.Generator().manual_seed(1), dtype=torch.float64).cuda()
+    a, va = job.jacobian("H2O", deterministic=True), job.jacobian("H2O", g_tau=g, deterministic=True)
+    assert all(torch.equal(x, y) for x, y in zip(a, job.jacobian("H2O", deterministic=True)))
+    seen, real = [], _lib.call
+
+    def no_cells(name, *args):
+        if name == "lbl_jacobian_ml_f32":
+            seen.append(args[-2] & _lib.LBL_LINE_CELLS)
+            args = args[:-2] + (args[-2] & ~_lib.LBL_LINE_CELLS, args[-1])
+        return real(name, *args)
+
+    monkeypatch.setattr(_lib, "call", no_cells)
+    b, vb = job.jacobian("H2O", deterministic=True), job.jacobian("H2O", g_tau=g, deterministic=True)
+    assert seen == [_lib.LBL_LINE_CELLS] * 2
+    for x, y in zip(a, b):
+        # truncation below 1e-8 of the cells' sums, two float32 evaluations a few 1e-7 apart
+        # (two leading terms of w' either way), per point against its layer's largest value
+        scale = y.abs().amax(dim=2, keepdim=True).clamp_min(1e-300)
+        assert ((x - y).abs() / scale).max().item() <= 2e-6
+        assert ((x.double() - y.double()).norm() / y.double().norm()).item() <= 2e-7
+    for x, y in zip(va, vb):
+        assert torch.all((x - y).abs() <= 2e-6 * y.abs().max())
+
+
 def test_geometries_without_cells(cuda):
     f = _lib.load().lbl_line_cells_floats
     assert f(3, 40_001, 2000, 0.001, 25.0) > 0
