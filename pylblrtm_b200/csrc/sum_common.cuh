@@ -28,6 +28,36 @@ __device__ __forceinline__ float rcp_approx(float v) {
   return r;
 }
 
+// Two float32 values per 64-bit register, one instruction for both (fma.rn.f32x2): the same
+// rounding as two fmaf, at the same multiply-add rate (71 TFLOP/s either way on B200) but half the
+// issue slots, which is what the summation kernels run out of.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ f32x2 dup2(float v) { return pack2(v, v); }
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// rcp_approx of both values.
+__device__ __forceinline__ f32x2 rcp2(f32x2 v) {
+  float a, b;
+  unpack2(v, a, b);
+  return pack2(rcp_approx(a), rcp_approx(b));
+}
+
 // Out-of-line general evaluations keep the register allocation of the hot
 // far-wing loop independent of the (rarely executed) full algorithm.
 static __device__ __noinline__ double re_w_f64(double x, double y) { return faddeeva<double>(x, y).re; }

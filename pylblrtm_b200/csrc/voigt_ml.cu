@@ -55,24 +55,6 @@ static __constant__ double c_dct16[ML_K * ML_K] = {LBL_DCT16};
 static __constant__ double c_dct8[ML_KF * ML_KF] = {LBL_DCT8};
 static_assert(ML_K == 16 && ML_KF == 8, "tables of cheb_tables.h");
 
-struct MlLine {
-  float4 g;   // jf (centre index relative to the chunk start), a, b, amp_far
-  float4 h;   // y, y^2, amp, value the clamped far-wing loop adds inside the near zone
-  float4 p;   // amp_far * (B_1, B_2, B_3, B_4)
-  float4 q;   // amp_far * (B_5, B_6, B_7, B_8)
-};
-
-// Re w times the line amplitude at one point, any distance (fast far wing first).
-__device__ __forceinline__ float line_value(float x, const MlLine& L) {
-  const float z2 = fmaf(x, x, L.h.y);
-  if (z2 >= FAR_Z2 && L.h.x >= 0.f) {
-    const float r = rcp_approx(z2);
-    return L.g.w * r * fmaf(fmaf(-2.0f * L.h.y, r, 1.5f), r, 1.0f);
-  }
-  if (z2 >= CORE_Z2 && L.h.x >= 0.f) return L.h.z * re_w_f32_mid(x, L.h.x, L.h.y, z2);
-  return (float)((double)L.h.z * weideman_re_f32((double)x, (double)L.h.x));
-}
-
 // Five-term asymptotic real part regrouped by powers of r = 1/|z|^2 for one line:
 // with s = y^2 (fixed per line) and q = s r, 1 + sum_k r^k A_k(q) = sum_m B_m(s) r^m,
 //   B_0 = 1, B_1 = 1.5, B_2 = 3.75 - 2s, B_3 = 13.125 - 15s, B_4 = 59.0625 - 105s + 12s^2,
@@ -94,29 +76,10 @@ __device__ __forceinline__ void asym5_line_coeffs(float s, float amp_far, float4
   }
 }
 
-// amp_far * S at r (the level-3 loop body without the final r factor).
-__device__ __forceinline__ float asym5_scaled(float r, const MlLine& R) {
-  float v = fmaf(R.q.w, r, R.q.z);
-  v = fmaf(v, r, R.q.y);
-  v = fmaf(v, r, R.q.x);
-  v = fmaf(v, r, R.p.w);
-  v = fmaf(v, r, R.p.z);
-  v = fmaf(v, r, R.p.y);
-  v = fmaf(v, r, R.p.x);
-  return fmaf(v, r, R.g.w);
-}
-
 // r = 1/|z|^2 with |z|^2 clamped to >= MID_Z2: inside the near zone the loop adds the
-// constant r_c * asym5_scaled(r_c), r_c = rcp(MID_Z2).
+// constant r_c * asym5_poly(r_c), r_c = rcp(MID_Z2).
 __device__ __forceinline__ float clamped_r(float x, float y2) {
   return rcp_approx(fmaxf(fmaf(x, x, y2), MID_Z2));
-}
-
-__device__ __forceinline__ void kahan_add(float& sum, float& comp, float v) {
-  const float yk = v - comp;
-  const float t = sum + yk;
-  comp = (t - sum) - yk;
-  sum = t;
 }
 
 // p(t) = c0/2 + sum_{k>=1} c_k T_k(t) by Clenshaw's recurrence (K coefficients).
@@ -131,6 +94,31 @@ __device__ __forceinline__ float clenshaw16(const float* c, float t) {
     b1 = b0;
   }
   return fmaf(t, b1, 0.5f * c[0] - b2);
+}
+
+// The same for K = 16 at P points (pairs), the coefficients' loop outside.
+template <int P>
+__device__ __forceinline__ void clenshaw_points(const float (&c)[ML_K], const f32x2 (&t)[P / 2], float (&v)[P]) {
+  f32x2 b1[P / 2], b2[P / 2], t2[P / 2];
+  const f32x2 neg = dup2(-1.0f), two = dup2(2.0f);
+#pragma unroll
+  for (int j = 0; j < P / 2; ++j) {
+    b1[j] = b2[j] = 0ull;
+    t2[j] = mul2(two, t[j]);
+  }
+#pragma unroll
+  for (int k = ML_K - 1; k >= 1; --k) {
+    const f32x2 ck = dup2(c[k]);
+#pragma unroll
+    for (int j = 0; j < P / 2; ++j) {
+      const f32x2 b0 = fma2(t2[j], b1[j], fma2(b2[j], neg, ck));
+      b2[j] = b1[j];
+      b1[j] = b0;
+    }
+  }
+  const f32x2 c0 = dup2(0.5f * c[0]);
+#pragma unroll
+  for (int j = 0; j < P / 2; ++j) unpack2(fma2(t[j], b1[j], fma2(b2[j], neg, c0)), v[2 * j], v[2 * j + 1]);
 }
 
 // ---------------------------------------------------------------------------
@@ -251,24 +239,42 @@ static __device__ __noinline__ float far_node_general(float x, float y, float y2
   return (float)((double)amp * weideman_re_f32_compact((double)x, (double)y));
 }
 
-// Node sums of one level-1 line: nodes k and K-1-k sit at +xs[k] and -xs[k] from the chunk centre.
+// Node sums of one level-1 line: nodes k and K-1-k (the halves of F[k]) sit at +xs[k] and -xs[k]
+// from the chunk centre.
 template <int K>
-__device__ __forceinline__ void far_line_nodes(float (&f)[K], const float (&xs)[K / 2], const LineF32& L, float xc,
+__device__ __forceinline__ void far_line_nodes(f32x2 (&F)[K / 2], const float (&xs)[K / 2], const LineF32& L, float xc,
                                                float y2, bool fast) {
   if (fast) {
-    const float ny2 = -2.0f * y2, na = -L.a;
+    const f32x2 ny2 = dup2(-2.0f * y2), a2 = dup2(L.a), xc2 = dup2(xc), y22 = dup2(y2), w = dup2(L.amp_far);
+    const f32x2 c1 = dup2(1.5f), c0 = dup2(1.0f);
 #pragma unroll
     for (int k = 0; k < K / 2; ++k) {
-      far_wing_add(f[k], fmaf(xs[k], L.a, xc), y2, ny2, L.amp_far);
-      far_wing_add(f[K - 1 - k], fmaf(xs[k], na, xc), y2, ny2, L.amp_far);
+      const f32x2 x = fma2(pack2(xs[k], -xs[k]), a2, xc2);
+      const f32x2 r = rcp2(fma2(x, x, y22));
+      F[k] = fma2(mul2(w, r), fma2(fma2(ny2, r, c1), r, c0), F[k]);
     }
   } else {
 #pragma unroll
     for (int k = 0; k < K / 2; ++k) {
-      f[k] += far_node_general(fmaf(xs[k], L.a, xc), L.y, y2, L.amp, L.amp_far);
-      f[K - 1 - k] += far_node_general(fmaf(xs[k], -L.a, xc), L.y, y2, L.amp, L.amp_far);
+      float a, b;
+      unpack2(F[k], a, b);
+      a += far_node_general(fmaf(xs[k], L.a, xc), L.y, y2, L.amp, L.amp_far);
+      b += far_node_general(fmaf(xs[k], -L.a, xc), L.y, y2, L.amp, L.amp_far);
+      F[k] = pack2(a, b);
     }
   }
+}
+
+// flush_nodes of paired node sums.
+template <int K>
+__device__ __forceinline__ void flush_pairs(f32x2 (&F)[K / 2], double* row, int lane) {
+  float f[K];
+#pragma unroll
+  for (int k = 0; k < K / 2; ++k) {
+    unpack2(F[k], f[k], f[K - 1 - k]);
+    F[k] = 0ull;
+  }
+  flush_nodes(f, row, lane);
 }
 
 __global__ void __launch_bounds__(MF_THREADS, 16)
@@ -307,11 +313,11 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
 #pragma unroll
   for (int k = 0; k < ML_KF / 2; ++k) xb[k] = H1 * c_node8[k];
 
-  float f1[ML_K], ff[ML_KF];
+  f32x2 f1[ML_K / 2], ff[ML_KF / 2];
 #pragma unroll
-  for (int k = 0; k < ML_K; ++k) f1[k] = 0.f;
+  for (int k = 0; k < ML_K / 2; ++k) f1[k] = 0ull;
 #pragma unroll
-  for (int k = 0; k < ML_KF; ++k) ff[k] = 0.f;
+  for (int k = 0; k < ML_KF / 2; ++k) ff[k] = 0ull;
   unsigned n1 = 0, nf = 0;
 
   // ---- the tile's lines split into cells to evaluate by their moments and other lines
@@ -398,14 +404,14 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
     }
     if (++rounds == MF_FLUSH) {                            // warp-uniform: every lane runs every round
       rounds = 0;
-      flush_nodes(f1, s_part[warp], lane);
-      flush_nodes(ff, s_part[warp] + ML_K, lane);
+      flush_pairs<ML_K>(f1, s_part[warp], lane);
+      flush_pairs<ML_KF>(ff, s_part[warp] + ML_K, lane);
     }
   }
   cp_async_wait<0>();                                      // only empty groups remain
   // node sums over the CTA in double: warps, then across warps
-  flush_nodes(f1, s_part[warp], lane);
-  flush_nodes(ff, s_part[warp] + ML_K, lane);
+  flush_pairs<ML_K>(f1, s_part[warp], lane);
+  flush_pairs<ML_KF>(ff, s_part[warp] + ML_K, lane);
   n1 = __reduce_add_sync(0xffffffffu, n1);
   nf = __reduce_add_sync(0xffffffffu, nf);
   __syncthreads();                                         // s_cnt zeroed, s_part written
@@ -452,8 +458,9 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
 //    sub-chunk from registers (node offsets are constant operands); the lanes' node
 //    sums are reduced once per round (transposed warp reduction) and added to the
 //    warp's float64 node sums;
-//  * level 3: each lane evaluates the line at its own 8 points, by the clamped
-//    five-term form, or by the two-term form when the line is far from every point of
+//  * level 3: each lane evaluates the line at its own 8 points, two per instruction
+//    (fma.rn.f32x2: whole spectrum 8.65 -> 8.05 ms, the series at the end in pairs too 8.00;
+//    pairs of level-2 nodes cost spills, 8.09), by the clamped five-term form, or by the two-term form when the line is far from every point of
 //    the sub-chunk (|z|^2 >= FAR_Z2 there);
 //  * near zones: the near points of the warp's level-3 lines inside its sub-chunk form
 //    an item space (middles, where the float64 core may apply, then tails); lanes take
@@ -487,6 +494,18 @@ __device__ __forceinline__ float asym5_poly(float r, float amp_far, const float4
   v = fmaf(v, r, p.y);
   v = fmaf(v, r, p.x);
   return fmaf(v, r, amp_far);
+}
+
+// The same at two values of r.
+__device__ __forceinline__ f32x2 asym5_poly2(f32x2 r, float amp_far, const float4& p, const float4& q) {
+  f32x2 v = fma2(dup2(q.w), r, dup2(q.z));
+  v = fma2(v, r, dup2(q.y));
+  v = fma2(v, r, dup2(q.x));
+  v = fma2(v, r, dup2(p.w));
+  v = fma2(v, r, dup2(p.z));
+  v = fma2(v, r, dup2(p.y));
+  v = fma2(v, r, dup2(p.x));
+  return fma2(v, r, dup2(amp_far));
 }
 
 // Level 2, one lane per line: lane i of each 32-line step takes line list[stride * i]
@@ -644,9 +663,9 @@ tau_ml_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restr
 
   // level-3 sums hold only the lines within ~2 sub-chunk widths (tens of terms), so
   // plain float accumulation suffices
-  float acc[P];
+  f32x2 acc[P / 2];                                          // points 2j and 2j + 1 of the lane
 #pragma unroll
-  for (int m = 0; m < P; ++m) acc[m] = 0.f;
+  for (int j = 0; j < P / 2; ++j) acc[j] = 0ull;
   unsigned long long n_pass = 0, n_nodes = 0, n_l3 = 0, n_near_items = 0;
 
   // register prefetch of the next round's line records
@@ -781,16 +800,24 @@ tau_ml_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restr
       const float x0 = fmaf(pl0 - g.x, g.y, -g.z);
       // |x| at the sub-chunk point nearest to the line centre (0 if it lies inside)
       const float xmin = fmaxf(fmaxf(fmaf(xw_lo - g.x, g.y, -g.z), -fmaf(xw_hi - g.x, g.y, -g.z)), 0.f);
+      const f32x2 a2 = dup2(g.y), x2 = dup2(x0), y2 = dup2(h.y);
       if (h.x >= 0.f && fmaf(xmin, xmin, h.y) >= FAR_Z2) {        // far from every point: two terms
-        const float ny2 = -2.0f * h.y;
+        const f32x2 ny2 = dup2(-2.0f * h.y), c1 = dup2(1.5f), c0 = dup2(1.0f), w = dup2(g.w);
 #pragma unroll
-        for (int m = 0; m < P; ++m) far_wing_add(acc[m], fmaf((float)m, g.y, x0), h.y, ny2, g.w);
+        for (int j = 0; j < P / 2; ++j) {
+          const f32x2 x = fma2(pack2((float)(2 * j), (float)(2 * j + 1)), a2, x2);
+          const f32x2 r = rcp2(fma2(x, x, y2));
+          acc[j] = fma2(mul2(w, r), fma2(fma2(ny2, r, c1), r, c0), acc[j]);
+        }
       } else {                                                    // |z|^2 clamped to >= MID_Z2
         const float4 p = s_p[l], q = s_q[l];
 #pragma unroll
-        for (int m = 0; m < P; ++m) {
-          const float r = clamped_r(fmaf((float)m, g.y, x0), h.y);
-          acc[m] = fmaf(r, asym5_poly(r, g.w, p, q), acc[m]);
+        for (int j = 0; j < P / 2; ++j) {
+          const f32x2 x = fma2(pack2((float)(2 * j), (float)(2 * j + 1)), a2, x2);
+          float z0, z1;
+          unpack2(fma2(x, x, y2), z0, z1);
+          const f32x2 r = pack2(rcp_approx(fmaxf(z0, MID_Z2)), rcp_approx(fmaxf(z1, MID_Z2)));
+          acc[j] = fma2(r, asym5_poly2(r, g.w, p, q), acc[j]);
         }
       }
     };
@@ -904,11 +931,14 @@ tau_ml_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restr
     // No barrier here: the next round stages into the other buffer.
   }
   __syncthreads();                                  // s_c1 visible even when no round ran
+  float l3[P];
+#pragma unroll
+  for (int j = 0; j < P / 2; ++j) unpack2(acc[j], l3[2 * j], l3[2 * j + 1]);
   if (n_w <= P) {                                   // lanes' level-3 sums at lane 0's points
 #pragma unroll
     for (int m = 0; m < P; ++m)
 #pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) acc[m] += __shfl_xor_sync(FULL_MASK, acc[m], o);
+      for (int o = 16; o >= 1; o >>= 1) l3[m] += __shfl_xor_sync(FULL_MASK, l3[m], o);
   }
 
   // ---- one Chebyshev series per sub-chunk: level-2 node sums + the 8-node interpolant
@@ -942,6 +972,16 @@ tau_ml_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restr
   }
   __syncwarp();
 
+  float series[P];
+  if (use_l2) {
+    f32x2 t[P / 2];
+#pragma unroll
+    for (int j = 0; j < P / 2; ++j) {
+      const int pl = w0 + lane * P + 2 * j;
+      t[j] = pack2(((float)pl - C2w) * inv_h2, ((float)(pl + 1) - C2w) * inv_h2);
+    }
+    clenshaw_points<P>(cw, t, series);
+  }
   const double T = t_layer[row];
   const float half_c2_t = (float)(0.5 * C2 / T);
   float* out = od + (long long)row * out_stride;   // points [out_first, out_first + out_stride) of the grid
@@ -953,13 +993,13 @@ tau_ml_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restr
       const long long p = c0 + pl;
       float v = s_core[pl - p0];
       if (use_l2) {
-        v += clenshaw16(cw, ((float)pl - C2w) * inv_h2);
+        v += series[m];
       } else if (use_l1) {
         const float t1 = ((float)pl - C1) * inv_h1;
         v += clenshaw16(s_c1, t1) + clenshaw16<ML_KF>(s_c1 + ML_K, t1);
       }
       const float nu = (float)grid_nu(nu_min, step, p);
-      const float o = (acc[m] + v) * (nu * tanhf(nu * half_c2_t));   // R(nu, T) = nu tanh(c2 nu / 2T)
+      const float o = (l3[m] + v) * (nu * tanhf(nu * half_c2_t));   // R(nu, T) = nu tanh(c2 nu / 2T)
       bad |= !isfinite(o);
       out[p - out_first] = o;
     }
