@@ -30,6 +30,8 @@
 // level-1 lines among them.
 #include <math.h>
 
+#include <type_traits>
+
 #include "cheb_tables.h"
 #include "faddeeva.cuh"
 #include "lbl_common.cuh"
@@ -45,7 +47,11 @@ constexpr int ML_CHUNK = ML_THREADS * ML_P;    // max points per CTA
 constexpr int ML_K = 16;                       // Chebyshev nodes per level
 constexpr int ML_KF = 8;                       // nodes for level-1 lines far from the chunk
 constexpr float ML_FAR1 = 3.f;                 // "far": more than (1 + ML_FAR1) half-widths from the centre
-constexpr float ML_MIN_H1 = 32.f;              // smallest chunk half-width (points) using level 1
+// Smallest chunk half-width (points) using level 1. A shorter chunk has at most P points, which
+// lanes share by lines; without level 1 one warp walks the whole window (5,000 lines) at every
+// point: the last 9 to 64 points of a grid took 790 us, tiles of 20 points 1,085 us where they now
+// take 35 and 64, and summed 5,000 float32 terms (od error 6e-6, 1.3e-5; now 1e-6, 1.7e-6).
+constexpr float ML_MIN_H1 = 4.f;
 constexpr float ML_MIN_H2 = 16.f;              // smallest sub-chunk half-width using level 2
 
 // Chebyshev node offsets (fractions of the half-width) and DCT weights, row-major [k][j]
@@ -586,23 +592,21 @@ __device__ __forceinline__ float near_correction(int p, const float4& g, const f
 }
 
 // One round's staged inner lines (slot = thread), in dynamic shared memory, two rounds deep.
+template <int ST>
 struct MlStage {
-  float4 g[ML_THREADS];            // jf, a, b, amp_far
-  float4 h[ML_THREADS];            // y, y^2, amp, clamped-loop value inside the near zone
-  float4 p[ML_THREADS];            // amp_far * (B_1 .. B_4)
-  float4 q[ML_THREADS];            // amp_far * (B_5 .. B_8)
-  short4 nr[ML_THREADS];           // near range (lo, n) and its middle (lo, n), chunk points
-  unsigned short cls[ML_THREADS];  // 2-bit class per warp: 0 -, 1 level 3, 2/3 level 2 (16/8)
+  float4 g[ST];            // jf, a, b, amp_far
+  float4 h[ST];            // y, y^2, amp, clamped-loop value inside the near zone
+  float4 p[ST];            // amp_far * (B_1 .. B_4)
+  float4 q[ST];            // amp_far * (B_5 .. B_8)
+  short4 nr[ST];           // near range (lo, n) and its middle (lo, n), chunk points
+  unsigned short cls[ST];  // 2-bit class per warp: 0 -, 1 level 3, 2/3 level 2 (16/8)
 };
-constexpr size_t ML_STAGE_BYTES = 2 * sizeof(MlStage);
 
-#ifndef LBL_ML_CTA_SUBS
-#define LBL_ML_CTA_SUBS 8
-#endif
-constexpr int ML_CTA_SUBS = LBL_ML_CTA_SUBS;    // 256-point sub-chunks (warps) per CTA of tau_ml_kernel
-
-template <bool DET>
-__global__ void __launch_bounds__(32 * ML_CTA_SUBS, 4 * 8 / ML_CTA_SUBS)
+// NW: 256-point sub-chunks (warps) per CTA, the chunk's; NW * 32 lines staged per round. Short
+// chunks get CTAs of their own size, so that as many warps share an SM as for long ones (a
+// 457-point tile in CTAs with 8 warps' buffers: 4 CTAs of 2 warps per SM).
+template <bool DET, int NW>
+__global__ void __launch_bounds__(32 * NW, 32 / NW)
 tau_ml_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restrict__ ranges,
               const int2* __restrict__ inner_ranges, const float* __restrict__ l1_work,
               const double* __restrict__ t_layer, double nu_min,
@@ -610,10 +614,9 @@ tau_ml_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restr
               int n_grp, float* __restrict__ od, int* err, unsigned long long* evals, unsigned long long* work,
               int tile_first, long long out_first, long long out_stride) {
   constexpr int P = ML_P;
-  constexpr int NW = ML_CTA_SUBS;
   constexpr int ST = 32 * NW;                       // lines staged per round (one per thread)
   extern __shared__ __align__(16) unsigned char s_dyn[];
-  MlStage* const s_stage = reinterpret_cast<MlStage*>(s_dyn);   // two rounds' staging buffers
+  MlStage<ST>* const s_stage = reinterpret_cast<MlStage<ST>*>(s_dyn);   // two rounds' staging buffers
   __shared__ unsigned char s_l2[NW][ST];    // per-warp level-2 slots (16 nodes from the front, 8 from the back)
   __shared__ unsigned char s_l3[NW][ST];    // per-warp level-3 slots
   __shared__ float s_core[NW * ML_WARP_PTS];        // near-zone corrections (each warp owns its points)
@@ -622,17 +625,13 @@ tau_ml_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restr
   __shared__ float s_nbuf[DET ? NW : 1][DET ? ML_NBW : 1];   // near-item values (bit-reproducible mode)
 
   const int row = blockIdx.y;
-  // a chunk's sub-chunks are split over `parts` CTAs of up to NW warps each
-  const int parts = (chunk_pts / ML_WARP_PTS + NW - 1) / NW;
-  const int chunk_id = blockIdx.x / parts, part = blockIdx.x % parts;
+  const int chunk_id = blockIdx.x;
   const int tile = tile_first + chunk_id / chunks_per_tile, chunk = chunk_id % chunks_per_tile;
   const long long t0 = (long long)tile * tile_samples;
   const long long t1 = min(t0 + (long long)tile_samples, n_nu);
   long long c0;
   int n_c;
   if (!tile_chunk(t0, t1, chunk, chunk_pts, c0, n_c)) return;
-  const int first_sub = part * NW, p0 = first_sub * ML_WARP_PTS;   // this CTA's first sub-chunk and point
-  if (p0 >= n_c) return;
   const int c0i = (int)c0;
   const double wlo = __dsub_rn(grid_nu(nu_min, step, t0), cutoff);
   const double whi = __dadd_rn(grid_nu(nu_min, step, t1 - 1), cutoff);
@@ -650,16 +649,16 @@ tau_ml_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restr
     rng = make_int2(max(rng.x, q.x), min(rng.y, q.y));
   }
   // this warp's sub-chunk
-  const int w0 = (first_sub + warp) * ML_WARP_PTS;
+  const int w0 = warp * ML_WARP_PTS;
   const int n_w = max(0, min(ML_WARP_PTS, n_c - w0));
   const float H2 = 0.5f * (float)(n_w - 1), C2w = (float)w0 + H2;
   const bool use_l2 = H2 >= ML_MIN_H2;
   const float pf = (float)(w0 + lane * P);                   // this lane's first point
 
-  for (int i = lane; i < ML_WARP_PTS; i += 32) s_core[w0 - p0 + i] = 0.f;
+  for (int i = lane; i < ML_WARP_PTS; i += 32) s_core[w0 + i] = 0.f;
   if (lane < ML_K + ML_KF) s_n2[warp][lane] = 0.0;
   if (use_l1 && tid < ML_K + ML_KF)
-    s_c1[tid] = l1_work[((long long)row * (gridDim.x / parts) + chunk_id) * (ML_K + ML_KF) + tid];
+    s_c1[tid] = l1_work[((long long)row * gridDim.x + chunk_id) * (ML_K + ML_KF) + tid];
 
   // level-3 sums hold only the lines within ~2 sub-chunk widths (tens of terms), so
   // plain float accumulation suffices
@@ -679,7 +678,7 @@ tau_ml_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restr
   if (tid * n_rounds < n_in) nxt = lp[rng.x + tid * n_rounds];
 
   for (int r = 0; r < n_rounds; ++r) {
-    MlStage& S = s_stage[r & 1];
+    MlStage<ST>& S = s_stage[r & 1];
     float4* const s_g = S.g;
     float4* const s_h = S.h;
     float4* const s_p = S.p;
@@ -700,10 +699,10 @@ tau_ml_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restr
     bool any3 = false;
     if (inner) {
       for (int w = 0; w < n_warps; ++w) {
-        const int nw = min(ML_WARP_PTS, n_c - (first_sub + w) * ML_WARP_PTS);
+        const int nw = min(ML_WARP_PTS, n_c - w * ML_WARP_PTS);
         if (nw <= 0) break;
         const float h2 = 0.5f * (float)(nw - 1);
-        const float d = fabsf(jf - ((float)((first_sub + w) * ML_WARP_PTS) + h2)) - h2;
+        const float d = fabsf(jf - ((float)(w * ML_WARP_PTS) + h2)) - h2;
         unsigned c = 1u;
         if (h2 >= ML_MIN_H2 && d > h2 + 1.f) c = d > ML_FAR1 * h2 ? 3u : 2u;
         any3 |= c == 1u;
@@ -888,7 +887,7 @@ tau_ml_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restr
             if (it0 + lane < total) {
               const float v = mid ? near_correction<true>(p, s_g[sl], s_h[sl])
                                   : near_correction<false>(p, s_g[sl], s_h[sl]);
-              if (v != 0.f) atomicAdd(&s_core[p - p0], v);
+              if (v != 0.f) atomicAdd(&s_core[p], v);
             }
           }
         }
@@ -919,7 +918,7 @@ tau_ml_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restr
               for (int it = ia + lane; it < ib; it += 32) {
                 const int k = it - st;
                 const int p = mid ? m_lo + k : (k < t_ln ? t_lo + k : t_hi + (k - t_ln));
-                s_core[p - p0] += s_nbuf[warp][it - b0];
+                s_core[p] += s_nbuf[warp][it - b0];
               }
               __syncwarp();
             }
@@ -991,7 +990,7 @@ tau_ml_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restr
     const int pl = w0 + lane * P + m;
     if (pl < n_c) {
       const long long p = c0 + pl;
-      float v = s_core[pl - p0];
+      float v = s_core[pl];
       if (use_l2) {
         v += series[m];
       } else if (use_l1) {
@@ -1006,7 +1005,7 @@ tau_ml_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __restr
   }
   if (bad) flag_error(err, row * (n_grp + 1) + n_grp);
   if (lane == 0 && evals && n_pass)
-    atomicAdd(evals, n_pass * (unsigned long long)(min(n_c, p0 + n_warps * ML_WARP_PTS) - p0));
+    atomicAdd(evals, n_pass * (unsigned long long)n_c);
   if (work) {   // work[0]: node evaluations, work[1]: level-3 loop evaluations, work[2]: near items
     if (n_nodes) atomicAdd(&work[0], n_nodes);
     if (n_l3) atomicAdd(&work[1], n_l3);
@@ -1091,9 +1090,7 @@ extern "C" int lbl_tau_tiles_ml_f32(const LineF32* prep, int n_lines, const int*
   long long chunks;
   ml_geometry(tile_samples, &threads, &cp, &chunks);
   const long long n_tiles = tile_count;
-  const int subs = threads / 32, parts = (subs + ML_CTA_SUBS - 1) / ML_CTA_SUBS;
-  const int cta_threads = 32 * (subs < ML_CTA_SUBS ? subs : ML_CTA_SUBS);
-  if (n_tiles * chunks * parts > 0x7fffffffLL) return lbl_set_error(LBL_EINVAL, "lbl_tau_tiles_ml_f32: grid too large");
+  if (n_tiles * chunks > 0x7fffffffLL) return lbl_set_error(LBL_EINVAL, "lbl_tau_tiles_ml_f32: grid too large");
   dim3 grid_far((unsigned)(n_tiles * chunks), (unsigned)n_rows);
   cudaStream_t st = (cudaStream_t)stream;
   // with LBL_LINE_CELLS the line cells follow the level-1 coefficients (16-byte aligned)
@@ -1108,27 +1105,28 @@ extern "C" int lbl_tau_tiles_ml_f32(const LineF32* prep, int n_lines, const int*
   tau_far_kernel<<<grid_far, MF_THREADS, 0, st>>>(prep, n_lines, (const int2*)ranges, nu_min, step, n_nu, tile_samples,
                                                    (int)chunks, cp, cutoff, l1_work, evals, work, tile_first, cg,
                                                    (const int*)cells, cells + cell_head(cg));
-  dim3 grid((unsigned)(n_tiles * chunks * parts), (unsigned)n_rows);
-  // the staging buffers take the kernel past 48 KB of shared memory: opt in (per call, so
-  // that every device and context the caller uses gets it; a host-side attribute write)
-  {
-    const void* fn = (flags & LBL_DETERMINISTIC) ? (const void*)tau_ml_kernel<true> : (const void*)tau_ml_kernel<false>;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ML_STAGE_BYTES);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  dim3 grid((unsigned)(n_tiles * chunks), (unsigned)n_rows);
+  auto launch = [&](auto kernel, size_t bytes) {
+    // the staging buffers can take the kernel past 48 KB of shared memory: opt in (per call, so
+    // that every device and context the caller uses gets it; a host-side attribute write)
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return lbl_set_error(LBL_ECUDA, "lbl_tau_tiles_ml_f32 (shared-memory attributes): %s", cudaGetErrorString(e));
     }
-  }
-  if (flags & LBL_DETERMINISTIC)
-    tau_ml_kernel<true><<<grid, cta_threads, ML_STAGE_BYTES, st>>>(prep, n_lines, (const int2*)ranges, (const int2*)inner, l1_work,
-                                                      t_layer, nu_min, step, n_nu, tile_samples, (int)chunks, cp,
-                                                      cutoff, n_grp, od, err, evals, work, tile_first, out_first,
-                                                      out_end - out_first);
-  else
-    tau_ml_kernel<false><<<grid, cta_threads, ML_STAGE_BYTES, st>>>(prep, n_lines, (const int2*)ranges, (const int2*)inner, l1_work,
-                                                       t_layer, nu_min, step, n_nu, tile_samples, (int)chunks, cp,
-                                                       cutoff, n_grp, od, err, evals, work, tile_first, out_first,
-                                                       out_end - out_first);
-  return lbl_check_launch("lbl_tau_tiles_ml_f32");
+    kernel<<<grid, threads, bytes, st>>>(prep, n_lines, (const int2*)ranges, (const int2*)inner, l1_work, t_layer, nu_min,
+                                         step, n_nu, tile_samples, (int)chunks, cp, cutoff, n_grp, od, err, evals, work,
+                                         tile_first, out_first, out_end - out_first);
+    return lbl_check_launch("lbl_tau_tiles_ml_f32");
+  };
+  auto by_size = [&](auto det) {
+    constexpr bool D = decltype(det)::value;
+    const int subs = threads / 32;
+    if (subs <= 1) return launch(tau_ml_kernel<D, 1>, 2 * sizeof(MlStage<32>));
+    if (subs <= 2) return launch(tau_ml_kernel<D, 2>, 2 * sizeof(MlStage<64>));
+    if (subs <= 4) return launch(tau_ml_kernel<D, 4>, 2 * sizeof(MlStage<128>));
+    return launch(tau_ml_kernel<D, 8>, 2 * sizeof(MlStage<256>));
+  };
+  return (flags & LBL_DETERMINISTIC) ? by_size(std::true_type()) : by_size(std::false_type());
 }

@@ -22,6 +22,8 @@
 // w' = -2zw + 2i/sqrt(pi) there would cancel catastrophically.
 #include <math.h>
 
+#include <type_traits>
+
 #include "cheb_tables.h"
 #include "faddeeva.cuh"
 #include "lbl_common.cuh"
@@ -35,7 +37,7 @@ constexpr int MJ_WARP_PTS = 32 * MJ_P;
 constexpr int MJ_THREADS = 256;
 constexpr int MJ_CHUNK = MJ_THREADS * MJ_P;       // 1024 points
 constexpr int MJ_K = 16;
-constexpr float MJ_MIN_H1 = 32.f;
+constexpr float MJ_MIN_H1 = 2.f;                   // shorter chunks (at most MJ_P points) use no level 1
 constexpr float MJ_MIN_H2 = 16.f;
 constexpr int MJ_NBW = 128;                        // near items buffered per warp (bit-reproducible mode)
 
@@ -539,8 +541,9 @@ jac_far_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__ jpr
   }
 }
 
-template <bool DET>
-__global__ void __launch_bounds__(MJ_THREADS, 3)
+// NW: warps (128-point sub-chunks) per CTA; short chunks get CTAs with buffers of their own size.
+template <bool DET, int NW>
+__global__ void __launch_bounds__(32 * NW, 24 / NW)
 jac_ml_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__ jprep, int n_lines,
               const int2* __restrict__ ranges, const int2* __restrict__ inner_ranges,
               const double* __restrict__ t_layer, double nu_min, double step, long long n_nu, int tile_samples,
@@ -548,16 +551,17 @@ jac_ml_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__ jpre
               float* __restrict__ d_t, float* __restrict__ d_v, int n_lay, const double* __restrict__ g_tau,
               double* __restrict__ vjp_t, double* __restrict__ vjp_v) {
   constexpr int P = MJ_P;
-  __shared__ JLine s2[MJ_THREADS];
-  __shared__ unsigned char s_l2[MJ_THREADS / 32][MJ_THREADS];
-  __shared__ unsigned char s_l3[MJ_THREADS / 32][MJ_THREADS];
-  __shared__ int s_cnt[MJ_THREADS / 32];
-  __shared__ short4 s_nr[MJ_THREADS];                // near range (lo, n) and its middle (lo, n), chunk points
-  __shared__ float s_core[3][MJ_CHUNK];              // near corrections (each warp owns its points)
+  constexpr int ST = 32 * NW;                        // lines staged per round (one per thread)
+  __shared__ JLine s2[ST];
+  __shared__ unsigned char s_l2[NW][ST];
+  __shared__ unsigned char s_l3[NW][ST];
+  __shared__ int s_cnt[NW];
+  __shared__ short4 s_nr[ST];                // near range (lo, n) and its middle (lo, n), chunk points
+  __shared__ float s_core[3][NW * MJ_WARP_PTS];              // near corrections (each warp owns its points)
   extern __shared__ float s_nbuf_dyn[];              // bit-reproducible mode: [warp][3][MJ_NBW] near-item values
   __shared__ float s_c1[MJ_NCOEF];                  // level-1 coefficients from jac_far_kernel
-  __shared__ float s_c2[MJ_THREADS / 32][3][MJ_K];   // merged series of levels 1 and 2 per warp
-  __shared__ double s_vjp[2][MJ_THREADS / 32];
+  __shared__ float s_c2[NW][3][MJ_K];   // merged series of levels 1 and 2 per warp
+  __shared__ double s_vjp[2][NW];
 
   const int row = blockIdx.y;
   const int tile = blockIdx.x / chunks_per_tile, chunk = blockIdx.x % chunks_per_tile;
@@ -591,7 +595,7 @@ jac_ml_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__ jpre
   const float xn2f = H2 * c_jnode8[lane & 7];
   const float pf = (float)(w0 + lane * P);
 
-  for (int i = tid; i < 3 * MJ_CHUNK; i += blockDim.x) (&s_core[0][0])[i] = 0.f;
+  for (int i = tid; i < 3 * NW * MJ_WARP_PTS; i += blockDim.x) (&s_core[0][0])[i] = 0.f;
 
   float acc[3][P];
 #pragma unroll
@@ -687,7 +691,7 @@ jac_ml_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__ jpre
       const unsigned q2f = __ballot_sync(0xffffffffu, is2f);
       const unsigned lt = (1u << lane) - 1u;
       if (is2) s_l2[warp][n2w + __popc(q2 & lt)] = (unsigned char)l;
-      if (is2f) s_l2[warp][MJ_THREADS - 1 - (n2fw + __popc(q2f & lt))] = (unsigned char)l;
+      if (is2f) s_l2[warp][ST - 1 - (n2fw + __popc(q2f & lt))] = (unsigned char)l;
       if (is3) s_l3[warp][n3w + __popc(q3 & lt)] = (unsigned char)l;
       n2w += __popc(q2);
       n2fw += __popc(q2f);
@@ -705,7 +709,7 @@ jac_ml_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__ jpre
       kahan3(sum2, comp2, a);
       // far level-2 lines: quarter-warps take one line each, lane (& 7) = node
       for (int i = lane >> 3; i < n2fw; i += 4) {
-        const JLine R = s2[s_l2[warp][MJ_THREADS - 1 - i]];
+        const JLine R = s2[s_l2[warp][ST - 1 - i]];
         const float x = fmaf(xn2f + (C2w - R.g.x), R.g.y, -R.g.z);
         add3(sum2f, value3(x, R), x, R);
       }
@@ -1065,25 +1069,27 @@ extern "C" int lbl_jacobian_ml_f32(const LineF32* prep, const LineJac* jprep, in
   jac_far_kernel<<<grid, MJF_THREADS, 0, st>>>(prep, jprep, n_lines, (const int2*)ranges, (const int2*)near, nu_min,
                                                step, n_nu, tile_samples, (int)chunks, cp, cutoff, l1_work, cg,
                                                (const int*)cells, cells + cell_head(cg));
-  if (flags & LBL_DETERMINISTIC) {
-    constexpr int dyn_bytes = (MJ_THREADS / 32) * 3 * MJ_NBW * (int)sizeof(float);   // near-item buffers
-    int dev = 0;
-    cudaGetDevice(&dev);
-    static int attr_set[64] = {0};
-    if (dev < 0 || dev >= 64) return lbl_set_error(LBL_EINVAL, "lbl_jacobian_ml_f32: device index out of range");
-    if (!attr_set[dev]) {
-      if (cudaFuncSetAttribute(jac_ml_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn_bytes) !=
-          cudaSuccess)
+  auto launch = [&](auto kernel, int nbuf_warps) {
+    // near-item buffers of the bit-reproducible mode (at most 12 KB)
+    kernel<<<grid, threads, nbuf_warps * 3 * MJ_NBW * sizeof(float), st>>>(
+        prep, jprep, n_lines, (const int2*)ranges, (const int2*)inner, t_layer, nu_min, step, n_nu, tile_samples,
+        (int)chunks, cutoff, l1_work, od, d_t, d_v, n_lay, g_tau, vjp_t, vjp_v);
+  };
+  auto by_size = [&](auto det) -> int {
+    constexpr bool D = decltype(det)::value;
+    const int nw = threads / 32;
+    if (D && nw > 4) {                              // with 8 warps' buffers past 48 KB of shared memory
+      if (cudaFuncSetAttribute(jac_ml_kernel<D, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               8 * 3 * MJ_NBW * (int)sizeof(float)) != cudaSuccess)
         return lbl_check_launch("lbl_jacobian_ml_f32 (shared memory attribute)");
-      attr_set[dev] = 1;
     }
-    jac_ml_kernel<true><<<grid, threads, dyn_bytes, st>>>(
-        prep, jprep, n_lines, (const int2*)ranges, (const int2*)inner, t_layer, nu_min, step, n_nu, tile_samples,
-        (int)chunks, cutoff, l1_work, od, d_t, d_v, n_lay, g_tau, vjp_t, vjp_v);
-  } else {
-    jac_ml_kernel<false><<<grid, threads, 0, st>>>(
-        prep, jprep, n_lines, (const int2*)ranges, (const int2*)inner, t_layer, nu_min, step, n_nu, tile_samples,
-        (int)chunks, cutoff, l1_work, od, d_t, d_v, n_lay, g_tau, vjp_t, vjp_v);
-  }
+    if (nw <= 1) launch(jac_ml_kernel<D, 1>, D ? 1 : 0);
+    else if (nw <= 2) launch(jac_ml_kernel<D, 2>, D ? 2 : 0);
+    else if (nw <= 4) launch(jac_ml_kernel<D, 4>, D ? 4 : 0);
+    else launch(jac_ml_kernel<D, 8>, D ? 8 : 0);
+    return LBL_OK;
+  };
+  const int rc = (flags & LBL_DETERMINISTIC) ? by_size(std::true_type()) : by_size(std::false_type());
+  if (rc != LBL_OK) return rc;
   return lbl_check_launch("lbl_jacobian_ml_f32");
 }
