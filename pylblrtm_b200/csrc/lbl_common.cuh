@@ -29,6 +29,28 @@ __device__ __forceinline__ void flag_error(int* err, int key) {
   if (err) atomicMin(err, key);
 }
 
+// Programmatic dependent launch: a kernel started with launch_dependent may begin while its
+// predecessor in the stream still runs. It calls dependency_wait before it touches global
+// memory (returns when the predecessor has finished and its writes are visible), and
+// dependency_trigger to let its own successor begin.
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dependency_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename K, typename... A>
+inline cudaError_t launch_dependent(K kernel, dim3 grid, int threads, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 }  // namespace lbl
 
 // Status plumbing of the C ABI (capi.cu).

@@ -294,6 +294,8 @@ gemm_bf16_kernel(const __grid_constant__ GemmOps<NB> ops, GemmGrid gg, int units
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  dependency_trigger();
+  dependency_wait();                           // operands of the kernels before
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
@@ -461,6 +463,8 @@ __global__ void __launch_bounds__(256)
 adam_group_kernel(const __grid_constant__ AdamGroup grp, int n, float lr, float b1, float b2, float eps, float c1,
                   float c2) {
   __shared__ __nv_bfloat16 s_t[ADAM_T][ADAM_T + 2];            // [column][row] of the tile
+  dependency_trigger();
+  dependency_wait();
   int k = 0;
   while (k + 1 < n && (int)blockIdx.x >= grp.first[k + 1]) ++k;
   const LblAdamItem& I = grp.it[k];
@@ -532,6 +536,8 @@ struct RowsumGroup {
 
 __global__ void __launch_bounds__(256)
 rowsum_group_kernel(const __grid_constant__ RowsumGroup grp, int n) {
+  dependency_trigger();
+  dependency_wait();
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= grp.first[n]) return;
   int k = 0;
@@ -588,6 +594,8 @@ struct PackGroup {
 
 __global__ void __launch_bounds__(256)
 pack_group_kernel(const __grid_constant__ PackGroup grp, const float* __restrict__ raw, int rows, int cols, int ld) {
+  dependency_trigger();
+  dependency_wait();
   const LblPackItem& I = grp.it[blockIdx.y];
   const int per = ld / 8;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -661,6 +669,8 @@ __global__ void __launch_bounds__(256)
 ensemble_gate4_kernel(const float4* __restrict__ pred, long long member_stride4, int ld4, int n_ch4,
                       const float* __restrict__ ch_scale, float scale, float gate, float4* __restrict__ mean,
                       float* __restrict__ est, int* __restrict__ flag) {
+  dependency_trigger();
+  dependency_wait();
   const int b = blockIdx.x;
   float worst = 0.0f;
   for (int c = threadIdx.x; c < n_ch4; c += blockDim.x) {
@@ -743,7 +753,9 @@ static int launch_gemm(const GemmOps<NB>& ops, int count, int M, int N, int K, i
   const long long units = (long long)gg.n_m * gg.n_n * n_split * count;
   if (units > 0x7fffffffLL) return lbl_set_error(LBL_EINVAL, "lbl_gemm_bf16: too many tiles");
   const int grid = (int)(units < n_sm ? units : n_sm);
-  gemm_bf16_kernel<BN, NB><<<grid, G_THREADS, GemmCfg<BN>::SMEM, stream>>>(ops, gg, (int)units, err);
+  // a layer's barriers, tensor memory and first instructions overlap the layer before
+  launch_dependent(gemm_bf16_kernel<BN, NB>, dim3((unsigned)grid), G_THREADS, GemmCfg<BN>::SMEM, stream, ops, gg,
+                   (int)units, err);
   return lbl_check_launch("lbl_gemm_bf16");
 }
 
@@ -857,7 +869,7 @@ extern "C" int lbl_adam_group(const LblAdamItem* items, int count, float lr, flo
       tiles += (long long)((g.it[i].rows + ADAM_T - 1) / ADAM_T) * ((g.it[i].cols + ADAM_T - 1) / ADAM_T);
       if (tiles > 0x7fffffffLL) return lbl_set_error(LBL_EINVAL, "lbl_adam_group: too many tiles");
     }
-    adam_group_kernel<<<(unsigned)tiles, 256, 0, (cudaStream_t)stream>>>(g, n, lr, b1, b2, eps, c1, c2);
+    launch_dependent(adam_group_kernel, dim3((unsigned)tiles), 256, 0, (cudaStream_t)stream, g, n, lr, b1, b2, eps, c1, c2);
     const int st = lbl_check_launch("lbl_adam_group");
     if (st != LBL_OK) return st;
   }
@@ -879,7 +891,7 @@ extern "C" int lbl_rowsum_group(const LblRowsumItem* items, int count, void* str
       if (rows > 0x7fffff00LL) return lbl_set_error(LBL_EINVAL, "lbl_rowsum_group: too many rows");
     }
     for (int i = n; i <= ROWSUM_ITEMS; ++i) g.first[i] = (int)rows;
-    rowsum_group_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, (cudaStream_t)stream>>>(g, n);
+    launch_dependent(rowsum_group_kernel, dim3((unsigned)((rows + 7) / 8)), 256, 0, (cudaStream_t)stream, g, n);
     const int st = lbl_check_launch("lbl_rowsum_group");
     if (st != LBL_OK) return st;
   }
@@ -900,7 +912,7 @@ extern "C" int lbl_pack_inputs_group(const float* raw, int rows, int cols, const
     }
     const long long t = (long long)rows * (ld / 8);
     dim3 grid((unsigned)((t + 255) / 256), (unsigned)n);
-    pack_group_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(g, raw, rows, cols, ld);
+    launch_dependent(pack_group_kernel, grid, 256, 0, (cudaStream_t)stream, g, raw, rows, cols, ld);
     const int st = lbl_check_launch("lbl_pack_inputs_group");
     if (st != LBL_OK) return st;
   }
@@ -933,8 +945,8 @@ extern "C" int lbl_ensemble_gate(const float* pred, int n_mem, long long member_
   const cudaStream_t st = (cudaStream_t)stream;
   const bool vec = n_ch % 4 == 0 && ld % 4 == 0 && member_stride % 4 == 0 && ((uintptr_t)pred | (uintptr_t)mean) % 16 == 0;
   auto vec_launch = [&](auto nm) {
-    ensemble_gate4_kernel<decltype(nm)::value><<<n_samples, 256, 0, st>>>(
-        (const float4*)pred, member_stride / 4, ld / 4, n_ch / 4, ch_scale, scale, gate, (float4*)mean, est, flag);
+    launch_dependent(ensemble_gate4_kernel<decltype(nm)::value>, dim3((unsigned)n_samples), 256, 0, st, (const float4*)pred,
+                     member_stride / 4, ld / 4, n_ch / 4, ch_scale, scale, gate, (float4*)mean, est, flag);
   };
   if (vec && n_mem == 2) vec_launch(std::integral_constant<int, 2>());
   else if (vec && n_mem == 3) vec_launch(std::integral_constant<int, 3>());
