@@ -151,7 +151,25 @@ __device__ __forceinline__ float gelu_grad(float z) {
   return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * __expf(-0.5f * z * z);
 }
 
-// 16 consecutive bf16 of one row: two 16-byte stores.
+// 32 bytes of one row: one store of a whole sector where the row is 32-byte aligned (the same for
+// all lanes of a warp: strides and bases decide it), else two of 16 bytes, which send every sector
+// to L2 twice. The rows of a warp lie in 32 different lines, so sectors are what the stores cost:
+// four members, 20,000 x 128 -> 1024 130 -> 120 us, 1024 -> 1024 204 -> 191, 1024 -> 2000 in
+// float32 414 -> 352 us (the products alone 22, 115 and 213 us; the GELU and the clock, which falls
+// to 1.6 GHz while tensor cores and epilogue both work, are the rest).
+__device__ __forceinline__ void store32(void* dst, const uint32_t* p) {
+  if (((uintptr_t)dst & 31) == 0) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(p[0]), "r"(p[1]),
+                 "r"(p[2]), "r"(p[3]), "r"(p[4]), "r"(p[5]), "r"(p[6]), "r"(p[7])
+                 : "memory");
+  } else {
+    uint4* d = reinterpret_cast<uint4*>(dst);
+    d[0] = make_uint4(p[0], p[1], p[2], p[3]);
+    d[1] = make_uint4(p[4], p[5], p[6], p[7]);
+  }
+}
+
+// 16 consecutive bf16 of one row.
 __device__ __forceinline__ void store_row16(__nv_bfloat16* dst, const float* v) {
   uint32_t p[8];
 #pragma unroll
@@ -159,9 +177,18 @@ __device__ __forceinline__ void store_row16(__nv_bfloat16* dst, const float* v) 
     __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
     p[i] = *reinterpret_cast<uint32_t*>(&h);
   }
-  uint4* d = reinterpret_cast<uint4*>(dst);
-  d[0] = make_uint4(p[0], p[1], p[2], p[3]);
-  d[1] = make_uint4(p[4], p[5], p[6], p[7]);
+  store32(dst, p);
+}
+
+// 16 consecutive floats of one row.
+__device__ __forceinline__ void store_row16(float* dst, const float* v) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t p[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) p[i] = __float_as_uint(v[8 * h + i]);
+    store32(dst + 8 * h, p);
+  }
 }
 
 // 16 bf16 of one row from memory (z_in of the GELU' epilogue).
@@ -182,10 +209,7 @@ __device__ __forceinline__ void load_row16(const __nv_bfloat16* src, float* v) {
 __device__ __forceinline__ void epilogue16(const LblGemmEpilogue& ep, int split, int row, int col, float* v,
                                            float& loss) {
   if (ep.mode == LBL_GEMM_F32) {
-    float4* d = reinterpret_cast<float4*>(ep.out_f32 + (long long)split * ep.split_stride +
-                                          (long long)row * ep.ld_f32 + col);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) d[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    store_row16(ep.out_f32 + (long long)split * ep.split_stride + (long long)row * ep.ld_f32 + col, v);
     return;
   }
   float bias[16];
@@ -210,11 +234,7 @@ __device__ __forceinline__ void epilogue16(const LblGemmEpilogue& ep, int split,
     float p[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) p[i] = __fdividef(1.0f, 1.0f + __expf(-(v[i] + bias[i])));
-    if (ep.out_f32) {
-      float4* d = reinterpret_cast<float4*>(ep.out_f32 + (long long)row * ep.ld_f32 + col);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) d[i] = make_float4(p[4 * i], p[4 * i + 1], p[4 * i + 2], p[4 * i + 3]);
-    }
+    if (ep.out_f32) store_row16(ep.out_f32 + (long long)row * ep.ld_f32 + col, p);
     if (!ep.target) return;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -332,6 +352,9 @@ gemm_bf16_kernel(const __grid_constant__ GemmOps<NB> ops, GemmGrid gg, int units
     }
   } else if (warp == 1) {
     if (lane == 0) {                           // MMA issuer
+      // one descriptor, advanced by adds: the lane shares its scheduler with four epilogue warps
+      // (1024 -> 1024 as above, built anew for each product: 191 against 188 us)
+      const uint64_t desc0 = sw128_desc(smem_u32(smem));
       int g = 0, i = 0;
       for (int u = blockIdx.x; u < units && !*fail; u += gridDim.x, ++i) {
         const int b = i & 1;
@@ -349,10 +372,10 @@ gemm_bf16_kernel(const __grid_constant__ GemmOps<NB> ops, GemmGrid gg, int units
             break;
           }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a0 = smem_u32(smem + s * Cfg::STAGE_BYTES), b0 = a0 + G_A_BYTES;
+          const uint64_t da = desc0 + (uint64_t)(s * (Cfg::STAGE_BYTES >> 4)), db = da + (G_A_BYTES >> 4);
 #pragma unroll
           for (int kk = 0; kk < GK / 16; ++kk)
-            umma_bf16(acc, sw128_desc(a0 + kk * 32), sw128_desc(b0 + kk * 32), Cfg::IDESC,
+            umma_bf16(acc, da + 2 * kk, db + 2 * kk, Cfg::IDESC,
                       (kt > 0 || kk > 0) ? 1u : 0u);
           umma_commit(smem_u32(&empty[s]));
         }

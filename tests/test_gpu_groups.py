@@ -151,3 +151,30 @@ def test_gate_kernels_agree(cuda, n_mem, n_ch):
         res.append((mean, est, flag))
     for x, y in zip(*res):
         assert _close_bits(x, y)
+
+
+# rows that start on 16 but not on 32 bytes take two stores each; the values are the same
+@pytest.mark.parametrize("m,n,k", [(128, 128, 64), (256, 512, 128)])
+def test_epilogue_rows_of_any_alignment(cuda, m, n, k):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    a, b = (torch.randn(s, generator=g, device="cuda").bfloat16() for s in ((m, k), (n, k)))
+    bias = torch.randn(n, generator=g, device="cuda")
+    ma, mb = surrogate._Map(a), surrogate._Map(b)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for mode, dt, step in ((_lib.GEMM_F32, torch.float32, 4), (_lib.GEMM_BIAS_SIGMOID, torch.float32, 4),
+                           (_lib.GEMM_BIAS_GELU, torch.bfloat16, 8)):
+        outs = []
+        for extra in (0, step, 2 * step):             # elements of 16, then 32 bytes more per row
+            buf = torch.full((m * (n + extra) + step,), -7.0, dtype=dt, device="cuda")
+            out = buf[step if extra else 0:][:m * (n + extra)].view(m, n + extra)
+            ep = _lib.GemmEpilogue()
+            ep.mode, ep.n_valid, ep.bias = mode, n, bias.data_ptr()
+            if dt == torch.float32:
+                ep.out_f32, ep.ld_f32 = out.data_ptr(), n + extra
+            else:
+                ep.y, ep.ld_y = out.data_ptr(), n + extra
+            _lib.call("lbl_gemm_bf16", ma.addr, mb.addr, m, n, k, 1, ctypes.addressof(ep), err.data_ptr(), _stream())
+            assert err.item() == 0
+            assert (out[:, n:] == -7.0).all()
+            outs.append(out[:, :n])
+        assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
