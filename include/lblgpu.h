@@ -391,6 +391,21 @@ typedef struct {
 } LblPackItem;
 int lbl_pack_inputs_group(const float* raw, int rows, int cols, const LblPackItem* items, int count, int ld,
                           void* stream);
+/* Predictions of the networks of an ensemble (one architecture: layer l is widths[l] -> widths[l+1],
+ * widths[0] the padded input width) on the same raw inputs [rows, n_in], rows <= M: the input pack,
+ * then each layer of all members in as few launches as fit. items and layers ([members][n_layers])
+ * hold what each member owns: normalisation and packed input, and per layer the maps of its input
+ * [M, widths[l]] and weights, its bias and its output y (bf16 [M, widths[l+1]]; not read for the
+ * last layer, which writes float32 [M, widths[n_layers]] to pred + member * member_stride). */
+typedef struct {
+  const void* map_x;
+  const void* map_w;
+  const float* bias;
+  void* y;
+} LblNetLayer;
+int lbl_ensemble_forward(const float* raw, int rows, int n_in, const LblPackItem* items, const LblNetLayer* layers,
+                         int members, int n_layers, const int* widths, int M, int n_valid, float* pred,
+                         long long member_stride, int* err, void* stream);
 /* out[r] = sum_c x[r, c] of a bf16 matrix (bias gradients). */
 int lbl_rowsum_bf16(const void* x, int rows, int cols, int ld, float* out, void* stream);
 /* Standardised bf16 network inputs: x[b, c] = (raw[b, c] - mean[c]) * inv_std[c] for

@@ -77,6 +77,7 @@ SIGNATURES = {
     "lbl_adam_group": (_I, [_P, _I, _F, _F, _F, _F, _I, _P]),
     "lbl_rowsum_group": (_I, [_P, _I, _P]),
     "lbl_pack_inputs_group": (_I, [_P, _I, _I, _P, _I, _I, _P]),
+    "lbl_ensemble_forward": (_I, [_P, _I, _I, _P, _P, _I, _I, _P, _I, _I, _P, _L, _P, _P]),
     "lbl_adam_step": (_I, [_P, _P, _P, _P, _I, _L, _I, _I, _I, _F, _F, _F, _F, _I, _P, _P, _I, _P]),
     "lbl_rowsum_bf16": (_I, [_P, _I, _I, _I, _P, _P]),
     "lbl_pack_inputs_bf16": (_I, [_P, _I, _I, _P, _P, _P, _I, _P, _I, _P]),
@@ -108,10 +109,6 @@ class RowsumItem(ctypes.Structure):
     """LblRowsumItem of include/lblgpu.h."""
     _fields_ = [("x", _P), ("out", _P), ("rows", _I), ("cols", _I), ("ld", _I), ("pad0", _I)]
 
-
-class PackItem(ctypes.Structure):
-    """LblPackItem of include/lblgpu.h."""
-    _fields_ = [("mean", _P), ("inv_std", _P), ("x", _P)]
 
 # host-side helpers (liblblio.so, include/lblio.h): no CUDA
 IO_LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "liblblio.so")

@@ -942,6 +942,45 @@ extern "C" int lbl_pack_inputs_group(const float* raw, int rows, int cols, const
   return LBL_OK;
 }
 
+// One host call for all launches of an ensemble's prediction: a handful of profiles is over on the
+// device before six calls with their argument blocks are made from outside (four members, 200
+// profiles: 100 us a pass when the host makes a call per layer, 69 us this way).
+extern "C" int lbl_ensemble_forward(const float* raw, int rows, int n_in, const LblPackItem* items,
+                                    const LblNetLayer* layers, int members, int n_layers, const int* widths, int M,
+                                    int n_valid, float* pred, long long member_stride, int* err, void* stream) {
+  if (!raw || !items || !layers || !widths || !pred || members < 1 || n_layers < 1 || rows < 1 || rows > M ||
+      member_stride < (long long)M * widths[n_layers])
+    return lbl_set_error(LBL_EINVAL, "lbl_ensemble_forward: bad arguments");
+  int st = lbl_pack_inputs_group(raw, rows, n_in, items, members, widths[0], stream);
+  for (int l = 0; l < n_layers && st == LBL_OK; ++l) {
+    const int k = widths[l], n = widths[l + 1];
+    for (int i0 = 0; i0 < members && st == LBL_OK; i0 += G_GROUP) {
+      const int count = members - i0 < G_GROUP ? members - i0 : G_GROUP;
+      const void *map_x[G_GROUP], *map_w[G_GROUP];
+      LblGemmEpilogue ep[G_GROUP] = {};
+      for (int i = 0; i < count; ++i) {
+        const LblNetLayer& L = layers[(long long)(i0 + i) * n_layers + l];
+        map_x[i] = L.map_x;
+        map_w[i] = L.map_w;
+        ep[i].bias = L.bias;
+        if (l < n_layers - 1) {
+          if (!L.y) return lbl_set_error(LBL_EINVAL, "lbl_ensemble_forward: member %d, layer %d: no output", i0 + i, l);
+          ep[i].mode = LBL_GEMM_BIAS_GELU;
+          ep[i].y = L.y;
+          ep[i].ld_y = n;
+        } else {
+          ep[i].mode = LBL_GEMM_BIAS_SIGMOID;
+          ep[i].n_valid = n_valid;
+          ep[i].out_f32 = pred + (i0 + i) * member_stride;
+          ep[i].ld_f32 = n;
+        }
+      }
+      st = lbl_gemm_bf16_group(count, map_x, map_w, M, n, k, ep, err, stream);
+    }
+  }
+  return st;
+}
+
 extern "C" int lbl_rowsum_bf16(const void* x, int rows, int cols, int ld, float* out, void* stream) {
   if (!x || !out || rows < 1 || cols < 1 || ld < cols)
     return lbl_set_error(LBL_EINVAL, "lbl_rowsum_bf16: bad arguments");

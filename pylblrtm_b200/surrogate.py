@@ -182,6 +182,7 @@ class _Workspace:
         self.raw = torch.zeros((batch, net.n_in), dtype=torch.float32, device=dev)
         self.x = [torch.zeros((batch, k), dtype=bf, device=dev) for k, _ in dims]
         self.map_x = [_Map(t) for t in self.x]
+        self.x_ptr = tuple(t.data_ptr() for t in self.x)
         self.train = train
         if train:
             self.xt = [torch.zeros((k, batch), dtype=bf, device=dev) for k, _ in dims]
@@ -508,7 +509,7 @@ class GatedSurrogate:
 
     def predictions(self, raw):
         """Every member's channel predictions [n_members, B, n_out] (device)."""
-        pred, B = self._members(raw)
+        pred, B, _ = self._members(raw)
         return pred[:, :B, :self.members[0].n_out]
 
     def _members(self, raw):
@@ -526,30 +527,19 @@ class GatedSurrogate:
             # the SMs for a handful of profiles and evens out the last wave of a large batch
             x = torch.broadcast_to(raw.detach(), (B, net0.n_in)).to(device=net0.dev, dtype=torch.float32).contiguous()
             wss = [n.workspace(Bp, False) for n in nets]
-            items = (_lib.PackItem * len(nets))(
-                *[_lib.PackItem(n.mean.data_ptr(), n.inv_std.data_ptr(), w.x[0].data_ptr()) for n, w in zip(nets, wss)])
-            _lib.call("lbl_pack_inputs_group", x.data_ptr(), B, net0.n_in, ctypes.addressof(items), len(nets),
-                      net0.dims[0][0], stream)
-            addrs = lambda maps: (ctypes.c_void_p * len(nets))(*[m.addr for m in maps])
-            for li, (k, n) in enumerate(net0.dims):
-                eps = (_lib.GemmEpilogue * len(nets))()
-                last = li == len(net0.dims) - 1
-                for m, (net, w) in enumerate(zip(nets, wss)):
-                    ep = eps[m]
-                    ep.bias = net.b[li].data_ptr()
-                    if last:
-                        ep.mode, ep.n_valid = _lib.GEMM_BIAS_SIGMOID, net.n_out
-                        ep.out_f32, ep.ld_f32 = pred.data_ptr() + 4 * m * Bp * n_pad, n
-                    else:
-                        ep.mode = _lib.GEMM_BIAS_GELU
-                        ep.y, ep.ld_y = w.x[li + 1].data_ptr(), n
-                _lib.call("lbl_gemm_bf16_group", len(nets), addrs(w.map_x[li] for w in wss),
-                          addrs(net.map_w[li] for net in nets), Bp, n, k, ctypes.addressof(eps),
-                          wss[0].err.data_ptr(), stream)
+            items, layers = [], []            # LblPackItem and LblNetLayer records, flat
+            for net, w in zip(nets, wss):
+                items += (net.mean.data_ptr(), net.inv_std.data_ptr(), w.x_ptr[0])
+                for mx, mw, b, y in zip(w.map_x, net.map_w, net.b, w.x_ptr[1:] + (0,)):
+                    layers += (mx.addr, mw.addr, b.data_ptr(), y)
+            widths = (ctypes.c_int * (len(net0.dims) + 1))(net0.dims[0][0], *[n for _, n in net0.dims])
+            _lib.call("lbl_ensemble_forward", x.data_ptr(), B, net0.n_in, (ctypes.c_void_p * len(items))(*items),
+                      (ctypes.c_void_p * len(layers))(*layers), len(nets), len(net0.dims), widths, Bp, net0.n_out,
+                      pred.data_ptr(), Bp * n_pad, wss[0].err.data_ptr(), stream)
             self.launches = -(-len(nets) // 16) + len(net0.dims) * -(-len(nets) // 8)
             for net in nets:
                 net.launches = 1 + len(net0.dims)
-            return pred, B
+            return pred, B, stream
         for m, net in enumerate(nets):
             ws = net.workspace(Bp, False)
             net.launches = 0
@@ -558,20 +548,20 @@ class GatedSurrogate:
                 ws.raw[B:].zero_()
             net._forward(ws, stream, False, out=pred[m])
             self.launches += net.launches
-        return pred, B
+        return pred, B, stream
 
     def ensemble(self, raw):
         """(mean [B, n_out], est [B], flag [B] bool) on the device."""
         torch = self.torch
         net0 = self.members[0]
-        pred, B = self._members(raw)
+        pred, B, stream = self._members(raw)
         Bp, n_pad = pred.shape[1], pred.shape[2]
         mean = torch.empty((B, net0.n_out), dtype=torch.float32, device=net0.dev)
         est = torch.empty((B,), dtype=torch.float32, device=net0.dev)
         flag = torch.empty((B,), dtype=torch.int32, device=net0.dev)
         _lib.call("lbl_ensemble_gate", pred.data_ptr(), len(self.members), Bp * n_pad, B, n_pad, net0.n_out,
                   _lib.ptr(self.ch_scale), self.scale, self.gate, mean.data_ptr(), est.data_ptr(), flag.data_ptr(),
-                  torch.cuda.current_stream().cuda_stream)
+                  stream)
         self.launches += 1
         return mean, est, flag.bool()
 
