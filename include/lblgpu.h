@@ -354,6 +354,10 @@ int lbl_gemm_bf16(const void* map_a, const void* map_b, int M, int N, int K, int
  * ensemble: product i is A_i . B_i^T with epilogue ep[i] (no split-K, no loss). */
 int lbl_gemm_bf16_group(int count, const void* const* map_a, const void* const* map_b, int M, int N, int K,
                         const LblGemmEpilogue* ep, int* err, void* stream);
+/* Two products of their own shapes (m, n, k, n_split: two values each) in one launch; neither reads
+ * what the other writes, and neither has a loss. */
+int lbl_gemm_bf16_pair(const void* const* map_a, const void* const* map_b, const int* m, const int* n, const int* k,
+                       const int* n_split, const LblGemmEpilogue* ep, int* err, void* stream);
 /* Adam (bias-corrected, step >= 1) on float32 master weights w [rows, cols] (row stride
  * ld) with moments m, v; the gradient is the in-order sum of n_split partials of g.
  * Refreshes the bf16 copy w_bf16 [rows, ld] and its transpose wt_bf16 [cols, ld_t]

@@ -74,6 +74,7 @@ SIGNATURES = {
     "lbl_tensor_map_bf16": (_I, [_P, _P, _L, _L, _L]),
     "lbl_gemm_bf16": (_I, [_P, _P, _I, _I, _I, _I, _P, _P, _P]),
     "lbl_gemm_bf16_group": (_I, [_I, _P, _P, _I, _I, _I, _P, _P, _P]),
+    "lbl_gemm_bf16_pair": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "lbl_adam_group": (_I, [_P, _I, _F, _F, _F, _F, _I, _P]),
     "lbl_rowsum_group": (_I, [_P, _I, _P]),
     "lbl_pack_inputs_group": (_I, [_P, _I, _I, _P, _I, _I, _P]),

@@ -260,19 +260,27 @@ __device__ __forceinline__ void epilogue16(const LblGemmEpilogue& ep, int split,
   }
 }
 
-// Work unit u -> (product, split, m tile, n tile); n varies fastest so concurrent CTAs share A.
+// Work units of a launch: unit -> (product, split, m tile, n tile); n varies fastest so
+// concurrent CTAs share A. One shape for all NB products, or two products (NB = 2) of their own
+// shapes, product i's units from first[i] on (a search over the products by every role cost an
+// ensemble of eight-product launches 2 to 8 %).
+template <int NB>
 struct GemmGrid {
-  int n_m, n_n, n_split, kt_per;
+  static constexpr int NS = NB == 2 ? 2 : 1;         // shapes
+  int n_m[NS], n_n[NS], n_split[NS], kt_per[NS], first[NS];
+  __device__ __forceinline__ int n_kt(int u) const { return kt_per[NS == 2 && u >= first[NS - 1]]; }
   __device__ __forceinline__ void unit(int u, int& op, int& split, int& m0, int& n0, int bn) const {
-    const int os = u / (n_m * n_n), r = u - os * n_m * n_n;
-    op = os / n_split;
-    split = os - op * n_split;
-    m0 = (r / n_n) * GM;
-    n0 = (r % n_n) * bn;
+    const int z = NS == 2 && u >= first[NS - 1];
+    if (z) u -= first[z];
+    const int os = u / (n_m[z] * n_n[z]), r = u - os * n_m[z] * n_n[z];
+    op = NS == 2 ? z : os / n_split[0];
+    split = NS == 2 ? os : os - op * n_split[0];
+    m0 = (r / n_n[z]) * GM;
+    n0 = (r % n_n[z]) * bn;
   }
 };
 
-// Operands of the NB products of one launch (same shapes).
+// Operands of the NB products of one launch.
 template <int NB>
 struct GemmOps {
   CUtensorMap a[NB], b[NB];
@@ -281,7 +289,7 @@ struct GemmOps {
 
 template <int BN, int NB>
 __global__ void __launch_bounds__(G_THREADS, 1)
-gemm_bf16_kernel(const __grid_constant__ GemmOps<NB> ops, GemmGrid gg, int units, int* err) {
+gemm_bf16_kernel(const __grid_constant__ GemmOps<NB> ops, const __grid_constant__ GemmGrid<NB> gg, int units, int* err) {
   using Cfg = GemmCfg<BN>;
   extern __shared__ unsigned char g_smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)g_smem_raw + 1023) & ~(uintptr_t)1023);
@@ -327,10 +335,10 @@ gemm_bf16_kernel(const __grid_constant__ GemmOps<NB> ops, GemmGrid gg, int units
       for (int u = blockIdx.x; u < units && !*fail; u += gridDim.x) {
         int op, split, m0, n0;
         gg.unit(u, op, split, m0, n0, BN);
-        const int k0 = split * gg.kt_per;
+        const int n_kt = gg.n_kt(u), k0 = split * n_kt;
         const CUtensorMap* map_a = &ops.a[NB == 1 ? 0 : op];
         const CUtensorMap* map_b = &ops.b[NB == 1 ? 0 : op];
-        for (int kt = 0; kt < gg.kt_per; ++kt, ++g) {
+        for (int kt = 0; kt < n_kt; ++kt, ++g) {
           const int s = g % GSTAGES;
           if (g >= GSTAGES && !mbar_wait(smem_u32(&empty[s]), ((g / GSTAGES) - 1) & 1)) {
             *fail = 1;
@@ -365,7 +373,8 @@ gemm_bf16_kernel(const __grid_constant__ GemmOps<NB> ops, GemmGrid gg, int units
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem + (uint32_t)(b * BN);
         bool ok = true;
-        for (int kt = 0; kt < gg.kt_per; ++kt, ++g) {
+        const int n_kt = gg.n_kt(u);
+        for (int kt = 0; kt < n_kt; ++kt, ++g) {
           const int s = g % GSTAGES;
           if (!mbar_wait(smem_u32(&full[s]), (g / GSTAGES) & 1)) {
             ok = false;
@@ -758,8 +767,10 @@ extern "C" int lbl_tensor_map_bf16(void* map_out, const void* base, long long ro
   return LBL_OK;
 }
 
+struct GemmSize { int M, N, K, n_split; };
+
 template <int BN, int NB>
-static int launch_gemm(const GemmOps<NB>& ops, int count, int M, int N, int K, int n_split, int n_sm, int dev, int* err,
+static int launch_gemm(const GemmOps<NB>& ops, const GemmSize* size, int count, int n_sm, int dev, int* err,
                        cudaStream_t stream) {
   static int attr_set[64] = {0};
   if (!attr_set[dev]) {
@@ -768,13 +779,18 @@ static int launch_gemm(const GemmOps<NB>& ops, int count, int M, int N, int K, i
       return lbl_check_launch("lbl_gemm_bf16 (shared memory attribute)");
     attr_set[dev] = 1;
   }
-  GemmGrid gg;
-  gg.n_m = M / GM;
-  gg.n_n = N / BN;
-  gg.n_split = n_split;
-  gg.kt_per = K / GK / n_split;
-  const long long units = (long long)gg.n_m * gg.n_n * n_split * count;
-  if (units > 0x7fffffffLL) return lbl_set_error(LBL_EINVAL, "lbl_gemm_bf16: too many tiles");
+  GemmGrid<NB> gg;
+  long long units = 0;
+  for (int i = 0; i < GemmGrid<NB>::NS; ++i) {
+    const GemmSize& z = size[i];
+    gg.n_m[i] = z.M / GM;
+    gg.n_n[i] = z.N / BN;
+    gg.n_split[i] = z.n_split;
+    gg.kt_per[i] = z.K / GK / z.n_split;
+    gg.first[i] = (int)units;
+    units += (long long)gg.n_m[i] * gg.n_n[i] * z.n_split * (GemmGrid<NB>::NS == 1 ? count : 1);
+    if (units > 0x7fffffffLL) return lbl_set_error(LBL_EINVAL, "lbl_gemm_bf16: too many tiles");
+  }
   const int grid = (int)(units < n_sm ? units : n_sm);
   // a layer's barriers, tensor memory and first instructions overlap the layer before
   launch_dependent(gemm_bf16_kernel<BN, NB>, dim3((unsigned)grid), G_THREADS, GemmCfg<BN>::SMEM, stream, ops, gg,
@@ -782,9 +798,9 @@ static int launch_gemm(const GemmOps<NB>& ops, int count, int M, int N, int K, i
   return lbl_check_launch("lbl_gemm_bf16");
 }
 
+// size: the shapes (one for all count products, or NB = 2 products' own).
 template <int NB>
-static int launch_group(const GemmOps<NB>& ops, int count, int M, int N, int K, int n_split, int* err,
-                        cudaStream_t stream) {
+static int launch_group(const GemmOps<NB>& ops, const GemmSize* size, int count, int* err, cudaStream_t stream) {
   int dev = 0;
   cudaGetDevice(&dev);
   static int n_sm[64] = {0};
@@ -793,9 +809,15 @@ static int launch_group(const GemmOps<NB>& ops, int count, int M, int N, int K, 
   // 256-wide tiles read a third less per product; 128-wide ones where 256-wide tiles would
   // leave more than a quarter of the SMs idle (4096 x 1024 x 1024, 128 wide tiles: 22.5 against
   // 24 us; four members of 256 x 2048 x 1024, 64 wide tiles: 17.2 against 12.5 us)
-  const long long wide = (long long)(M / GM) * (N / 256) * n_split * count;
-  if (N % 256 == 0 && 4 * wide >= 3 * n_sm[dev]) return launch_gemm<256, NB>(ops, count, M, N, K, n_split, n_sm[dev], dev, err, stream);
-  return launch_gemm<128, NB>(ops, count, M, N, K, n_split, n_sm[dev], dev, err, stream);
+  long long wide = 0;
+  bool fits = true;
+  constexpr int NS = GemmGrid<NB>::NS;
+  for (int i = 0; i < NS; ++i) {
+    wide += (long long)(size[i].M / GM) * (size[i].N / 256) * size[i].n_split * (NS == 1 ? count : 1);
+    fits = fits && size[i].N % 256 == 0;
+  }
+  if (fits && 4 * wide >= 3 * n_sm[dev]) return launch_gemm<256, NB>(ops, size, count, n_sm[dev], dev, err, stream);
+  return launch_gemm<128, NB>(ops, size, count, n_sm[dev], dev, err, stream);
 }
 
 static int check_gemm(const void* map_a, const void* map_b, int M, int N, int K, int n_split,
@@ -825,7 +847,31 @@ extern "C" int lbl_gemm_bf16(const void* map_a, const void* map_b, int M, int N,
   memcpy(&ops.a[0], map_a, sizeof(CUtensorMap));
   memcpy(&ops.b[0], map_b, sizeof(CUtensorMap));
   ops.ep[0] = *ep;
-  return launch_group<1>(ops, 1, M, N, K, n_split, err, (cudaStream_t)stream);
+  const GemmSize size = {M, N, K, n_split};
+  return launch_group<1>(ops, &size, 1, err, (cudaStream_t)stream);
+}
+
+// Two products of their own shapes in one launch. A training step's layers are one wave of tiles
+// each, so a launch of one product ends with an epilogue that nothing overlaps; a layer's weight
+// gradient (split over the batch) and its input gradient need the same operand and not each other
+// (four steps of a 61-1024x4-2000 network at batch 4,096: 1,740 us as two launches, 1,660 together).
+extern "C" int lbl_gemm_bf16_pair(const void* const* map_a, const void* const* map_b, const int* m, const int* n,
+                                  const int* k, const int* n_split, const LblGemmEpilogue* ep, int* err,
+                                  void* stream) {
+  if (!map_a || !map_b || !m || !n || !k || !n_split || !ep)
+    return lbl_set_error(LBL_EINVAL, "lbl_gemm_bf16_pair: bad arguments");
+  GemmOps<2> ops;
+  GemmSize size[2];
+  for (int i = 0; i < 2; ++i) {
+    const int st = check_gemm(map_a[i], map_b[i], m[i], n[i], k[i], n_split[i], ep + i);
+    if (st != LBL_OK) return st;
+    if (ep[i].loss) return lbl_set_error(LBL_EINVAL, "lbl_gemm_bf16_pair: no loss in a pair");
+    memcpy(&ops.a[i], map_a[i], sizeof(CUtensorMap));
+    memcpy(&ops.b[i], map_b[i], sizeof(CUtensorMap));
+    ops.ep[i] = ep[i];
+    size[i] = {m[i], n[i], k[i], n_split[i]};
+  }
+  return launch_group<2>(ops, size, 2, err, (cudaStream_t)stream);
 }
 
 constexpr int G_GROUP = 8;   // products per launch (3.1 KB of kernel parameters)
@@ -841,13 +887,14 @@ extern "C" int lbl_gemm_bf16_group(int count, const void* const* map_a, const vo
   for (int i0 = 0; i0 < count; i0 += G_GROUP) {
     const int n = count - i0 < G_GROUP ? count - i0 : G_GROUP;
     GemmOps<G_GROUP> ops;
+    const GemmSize size = {M, N, K, 1};
     for (int i = 0; i < G_GROUP; ++i) {               // unused entries repeat the first
       const int j = i0 + (i < n ? i : 0);
       memcpy(&ops.a[i], map_a[j], sizeof(CUtensorMap));
       memcpy(&ops.b[i], map_b[j], sizeof(CUtensorMap));
       ops.ep[i] = ep[j];
     }
-    const int st = launch_group<G_GROUP>(ops, n, M, N, K, 1, err, (cudaStream_t)stream);
+    const int st = launch_group<G_GROUP>(ops, &size, n, err, (cudaStream_t)stream);
     if (st != LBL_OK) return st;
   }
   return LBL_OK;

@@ -355,17 +355,23 @@ class MLP:
         for li in range(len(self.dims) - 1, -1, -1):
             k, n = self.dims[li]
             s = ws.split[li]
-            ep = _lib.GemmEpilogue()
-            ep.mode = _lib.GEMM_F32
-            ep.out_f32, ep.ld_f32, ep.split_stride = ws.dw[li].data_ptr(), k, n * k
-            self._gemm(ws.map_dzt[li], ws.map_xt[li], n, k, B, ep, ws, stream, n_split=s)
-            if li > 0:
-                ep = _lib.GemmEpilogue()
-                ep.mode = _lib.GEMM_DGELU
-                ep.z_in, ep.ld_zin = ws.z[li - 1].data_ptr(), k
-                ep.y, ep.ld_y = ws.dz[li - 1].data_ptr(), k
-                ep.y_t, ep.ld_yt = ws.dzt[li - 1].data_ptr(), B
-                self._gemm(ws.map_dz[li], self.map_wt[li], B, k, n, ep, ws, stream)
+            # the weight gradient and, below the first layer, the input gradient of the same dz
+            ep = (_lib.GemmEpilogue * 2)()
+            ep[1].mode = _lib.GEMM_F32
+            ep[1].out_f32, ep[1].ld_f32, ep[1].split_stride = ws.dw[li].data_ptr(), k, n * k
+            if li == 0:
+                self._gemm(ws.map_dzt[0], ws.map_xt[0], n, k, B, ep[1], ws, stream, n_split=s)
+                break
+            ep[0].mode = _lib.GEMM_DGELU
+            ep[0].z_in, ep[0].ld_zin = ws.z[li - 1].data_ptr(), k
+            ep[0].y, ep[0].ld_y = ws.dz[li - 1].data_ptr(), k
+            ep[0].y_t, ep[0].ld_yt = ws.dzt[li - 1].data_ptr(), B
+            two = ctypes.c_int * 2
+            addrs = ctypes.c_void_p * 2
+            _lib.call("lbl_gemm_bf16_pair", addrs(ws.map_dz[li].addr, ws.map_dzt[li].addr),
+                      addrs(self.map_wt[li].addr, ws.map_xt[li].addr), two(B, n), two(k, k), two(n, B), two(1, s),
+                      ctypes.addressof(ep), ws.err.data_ptr(), stream)
+            self.launches += 1
         items = (_lib.RowsumItem * len(self.dims))(
             *[_lib.RowsumItem(ws.dzt[li].data_ptr(), ws.db[li].data_ptr(), n, B, B) for li, (_, n) in
               enumerate(self.dims)])

@@ -178,3 +178,38 @@ def test_epilogue_rows_of_any_alignment(cuda, m, n, k):
             assert (out[:, n:] == -7.0).all()
             outs.append(out[:, :n])
         assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+# two products of their own shapes: 256-wide tiles, 128-wide ones, unequal depths and split-K
+@pytest.mark.parametrize("shapes", [[(4096, 1024, 1024, 1), (1024, 1024, 4096, 4)], [(128, 128, 64, 1), (128, 128, 128, 2)],
+                                    [(384, 384, 256, 1), (128, 512, 1024, 8)], [(256, 256, 192, 1), (128, 128, 64, 1)]])
+def test_gemm_pair_equals_single(cuda, shapes):
+    g = torch.Generator(device="cuda").manual_seed(len(shapes) + shapes[0][0])
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    ab = [(rnd(m, k).bfloat16(), rnd(n, k).bfloat16()) for m, n, k, _ in shapes]
+    maps = [(surrogate._Map(a), surrogate._Map(b)) for a, b in ab]
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    (m0, n0, _, _), (m1, n1, _, s1) = shapes
+    z = rnd(m0, n0).bfloat16()
+    outs, eps = [], []
+    for _ in range(2):
+        o = [torch.zeros((m0, n0), dtype=torch.bfloat16, device="cuda"),
+             torch.zeros((n0, m0), dtype=torch.bfloat16, device="cuda"), torch.zeros((s1, m1, n1), device="cuda")]
+        ep = (_lib.GemmEpilogue * 2)()
+        ep[0].mode, ep[0].z_in, ep[0].ld_zin = _lib.GEMM_DGELU, z.data_ptr(), n0
+        ep[0].y, ep[0].ld_y, ep[0].y_t, ep[0].ld_yt = o[0].data_ptr(), n0, o[1].data_ptr(), m0
+        ep[1].mode, ep[1].out_f32, ep[1].ld_f32, ep[1].split_stride = _lib.GEMM_F32, o[2].data_ptr(), n1, m1 * n1
+        outs.append(o)
+        eps.append(ep)
+    for i, (m, n, k, s) in enumerate(shapes):
+        _lib.call("lbl_gemm_bf16", maps[i][0].addr, maps[i][1].addr, m, n, k, s, ctypes.addressof(eps[0][i]),
+                  err.data_ptr(), _stream())
+    ptrs = lambda j: (ctypes.c_void_p * 2)(*[p[j].addr for p in maps])
+    ints = lambda j: (ctypes.c_int * 2)(*[s[j] for s in shapes])
+    _lib.call("lbl_gemm_bf16_pair", ptrs(0), ptrs(1), ints(0), ints(1), ints(2), ints(3), ctypes.addressof(eps[1]),
+              err.data_ptr(), _stream())
+    assert err.item() == 0
+    for x, y in zip(*outs):
+        assert torch.equal(x, y) and x.float().abs().sum() > 0
+    want = (ab[1][0].float() @ ab[1][1].float().T)                      # the split sums are the product
+    assert torch.allclose(outs[1][2].sum(0), want, rtol=1e-4, atol=1e-4 * shapes[1][2] ** 0.5)
