@@ -40,20 +40,20 @@ UNIT = "line-evals/s"
 WORKLOAD = "three_gas_200k_lines_60_layers_600-2500cm-1_step0.001_cutoff25_tile2_mu0.8"
 FLOPS_PER_EVAL_FAR = 12      # two-term far-wing form: 5 FFMA + 1 FMUL + 1 RCP (FMA = 2 flops)
 # multi-level kernel, per unit of each work category (FMA = 2 flops, RCP = 1):
-FLOPS_NODE = 12              # Chebyshev-node evaluation (two-term form)
+FLOPS_NODE = 12              # Chebyshev-node evaluation (two-term form; a line cell counts as two)
 FLOPS_L3 = 24                # level-3 loop evaluation (clamped five-term form by powers of 1/|z|^2: 2 FMA + max + RCP + 9 FMA)
 FLOPS_NEAR = 60              # near-zone point (float continued fraction / float64 rational, average)
 FLOPS_CHEB_PER_POINT = 144   # 16 + 8 Clenshaw terms for each of levels 1 and 2 (3 flops a term)
 CPU_SAMPLE = (1000.0, 1000.5)  # sub-window timed on the host (all 60 layers)
 
 
-# DRAM traffic of one lbl_tau_tiles_ml_f32 call on the default workload (200k lines, 60
-# layers, 600-2500 cm^-1), from a single-pass ncu capture of its two launches
-# (profiles/launches_three_gas_200k_fp32_ml.md): tau_far_kernel 384.53 MB read + 7.91 MB
-# written, tau_ml_kernel 391.63 MB read + 451.51 MB written. Each kernel reads the 384 MB
-# of line records once; tau_ml_kernel writes the 456 MB optical depth (part of it still in
-# L2 when the launch ends).
-TAU_ML_DRAM_BYTES = 384.532480e6 + 7.905280e6 + 391.629568e6 + 451.512064e6
+# DRAM traffic of the summation (lbl_line_cells and lbl_tau_tiles_ml_f32) on the default
+# workload (200k lines, 60 layers, 600-2500 cm^-1), from a single-pass ncu capture of its
+# three large launches (profiles/launches_three_gas_200k_fp32_ml.md): line_moments_kernel
+# 384.19 MB read + 14.70 MB written, tau_far_kernel 398.75 + 5.12 MB, tau_ml_kernel 391.30 +
+# 450.48 MB. Each kernel reads the 384 MB of line records once; tau_ml_kernel writes the
+# 456 MB optical depth (part of it still in L2 when the launch ends).
+TAU_ML_DRAM_BYTES = 384.189440e6 + 14.696448e6 + 398.746880e6 + 5.123072e6 + 391.298560e6 + 450.483456e6
 
 
 def parse():
@@ -288,22 +288,21 @@ def _timed_ms(torch, fn, reps):
 def plain_and_accuracy(torch, job, sd, prof, grid, evals, fp32_value):
     """The comparison engines and the accuracy of the default one, on the full workload.
 
-    (1) The plain float64 method (every admitted line at every point, Gautschi-type
-    Faddeeva in float64, the reference's ``_voigt``/``phi @ S`` work done directly) and
-    the direct float32 method: line-evals/s from CUDA-event times of whole spectra, and
-    the default engine's ratio to each. (2) The default float32 engine against the
-    float64 engine on the full 200k-line, 60-layer, 1.9M-point spectrum at full
-    strength (saturated: T ~ 0 almost everywhere) and with line strengths x 1e-3 and
-    x 1e-5, where T spans (0, 1) and |dT| tests something. (3) Both engines against the
-    reference's own outputs (golden vectors made by running the reference) for the
-    2,000-line CO2 band at full strength and x 1e-3.
+    (1) The float64 engine (three Chebyshev levels at float64 accuracy) and the direct
+    float32 method (every admitted line at every point): line-evals/s from CUDA-event
+    times of whole spectra, and the default engine's ratio to each. (2) The default
+    float32 engine against the float64 engine on the full 200k-line, 60-layer,
+    1.9M-point spectrum at full strength (saturated: T ~ 0 almost everywhere) and with
+    line strengths x 1e-3 and x 1e-5, where T spans (0, 1) and |dT| tests something.
+    (3) Both engines against the reference's own outputs (golden vectors made by running
+    the reference) for the 2,000-line CO2 band at full strength and x 1e-3.
     """
     from pylblrtm_b200 import engine, synthetic
     out_plain, acc = {}, {}
     run = lambda j, prec: j.run(prec, mu=[0.8], want_od=False, want_tau=True, want_trans=True)
     r64 = run(job, "fp64")                                   # also the float64 warm-up
-    ms64 = _timed_ms(torch, lambda: job.run("fp64", mu=[0.8], want_od=False, want_trans=True), 1)
-    out_plain["fp64_plain"] = {"ms_per_spectrum": ms64, "line_evals_per_s": evals / (ms64 * 1e-3), "steps": 1,
+    ms64 = _timed_ms(torch, lambda: job.run("fp64", mu=[0.8], want_od=False, want_trans=True), 2)
+    out_plain["fp64"] = {"ms_per_spectrum": ms64, "line_evals_per_s": evals / (ms64 * 1e-3), "steps": 2,
                                "kernel": "tau_f64_kernel (lbl_tau_tiles_f64)"}
     r32 = run(job, "fp32")
     acc["three_gas_200k_fp32_vs_fp64"] = _errors(torch, r32.trans[0], r64.trans[0], r32.tau[0], r64.tau[0])
@@ -312,7 +311,7 @@ def plain_and_accuracy(torch, job, sd, prof, grid, evals, fp32_value):
     out_plain["fp32_direct"] = {"ms_per_spectrum": msd, "line_evals_per_s": evals / (msd * 1e-3), "steps": 2,
                                 "kernel": "tau_f32_kernel (lbl_tau_tiles_f32)"}
     acc["three_gas_200k_fp32_direct_vs_fp64"] = _errors(torch, rd.trans[0], r64.trans[0], rd.tau[0], r64.tau[0])
-    out_plain["fp32_over_fp64"] = fp32_value / out_plain["fp64_plain"]["line_evals_per_s"]
+    out_plain["fp32_over_fp64"] = fp32_value / out_plain["fp64"]["line_evals_per_s"]
     out_plain["fp32_over_direct"] = fp32_value / out_plain["fp32_direct"]["line_evals_per_s"]
     del r64, r32, rd
     for scale in (1e-3, 1e-5):
@@ -609,11 +608,12 @@ def main():
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak,
                      "traffic": TAU_ML_DRAM_BYTES if (a.precision == "fp32" and full_size and world == 1) else None,
-                     "traffic_unit": "bytes per call of both kernels (ncu dram__bytes_read.sum + dram__bytes_write.sum)",
+                     "traffic_unit": "bytes per call of the three kernels (ncu dram__bytes_read.sum + dram__bytes_write.sum)",
                      "algorithmic_bytes": r0_lines_bytes + job.n_prof * job.n_lay * n_out * 4,
                      "algorithmic_bytes_rule": "32-B prepared line record per (layer, line) read once + "
                                                "float32 od written once per (layer, point)",
-                     "kernel": {"fp32": "tau_far_kernel + tau_ml_kernel<0> (one lbl_tau_tiles_ml_f32 call)",
+                     "kernel": {"fp32": "line_moments_kernel + tau_far_kernel + tau_ml_kernel<0> "
+                                        "(lbl_line_cells and one lbl_tau_tiles_ml_f32 call)",
                                 "fp32-direct": "tau_f32_kernel",
                                 "fp64": "tau_f64_kernel"}[a.precision],
                      "faddeeva_evals_per_launch": work_per_step,

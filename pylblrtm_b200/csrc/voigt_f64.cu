@@ -10,7 +10,7 @@
 // line's own value is below 16 * 11.9^-16 ~ 1e-16 (its slope in a 1/x^2 wing included), so
 // the sums keep float64 accuracy; interpolants are evaluated at the rounded grid values
 // themselves. Three interval sizes share the work of one CTA (256 threads, one chunk of at
-// most 1,024 points of one tile of one row):
+// most 512 points of one tile of one row):
 //   level 1  the chunk: one thread takes one line and adds it at the 16 nodes;
 //   level 2  256-point sub-chunks, one after the other: the lines that are not far of the
 //            chunk, again one per thread; those not far of the sub-chunk go to a list;
@@ -18,8 +18,8 @@
 //            lane; the remaining lines directly, one point per lane.
 // A far line also needs |z|^2 >= ASYM_Z2 at its nearest node, so every node value is the
 // asymptotic series in its real-part form with one reciprocal; what fails that test is
-// summed directly at each point (longer series, Weideman's approximation in the core). Every sum is formed in a fixed order (no floating-point atomics), so
-// results are bit-reproducible.
+// summed directly at each point (longer series, Weideman's approximation in the core). Every
+// sum is formed in a fixed order (no floating-point atomics), so results are bit-reproducible.
 //
 // Bound by float64 issue and latency (two CTAs per SM at 128 registers): about 240 node
 // values and 20 direct values per point and layer at 105 lines per cm^-1, 0.001 cm^-1 steps
