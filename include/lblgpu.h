@@ -416,6 +416,12 @@ int lbl_rowsum_bf16(const void* x, int rows, int cols, int ld, float* out, void*
  * c < cols, zero up to ld; the transposed copy x_t [ld, ld_t] when non-NULL. */
 int lbl_pack_inputs_bf16(const float* raw, int rows, int cols, const float* mean, const float* inv_std, void* x,
                          int ld, void* x_t, int ld_t, void* stream);
+/* A training batch from samples idx [rows] (int64, each in [0, n_samples); others become NaN) of
+ * features [n_samples, n_in] and targets [n_samples, n_out]: x and x_t as lbl_pack_inputs_bf16 of the
+ * selected rows, the targets' rows, *loss = 0. One launch. */
+int lbl_stage_batch(const float* features, const float* targets, const long long* idx, long long n_samples, int rows,
+                    int n_in, int n_out, const float* mean, const float* inv_std, void* x, int ld, void* x_t, int ld_t,
+                    float* target, double* loss, void* stream);
 /* Ensemble gate: for each sample b, mean[b, c] over the n_mem members' predictions
  * pred[m * member_stride + b * ld + c], est[b] = max_c of their standard deviation,
  * weighted by ch_scale[c] when ch_scale (device, [n_ch]) is not NULL, and

@@ -319,15 +319,17 @@ class MLP:
                   ws.err.data_ptr(), stream)
         self.launches += 1
 
-    def _forward(self, ws: _Workspace, stream, train: bool, out=None) -> None:
+    def _forward(self, ws: _Workspace, stream, train: bool, out=None, packed: bool = False) -> None:
         """Forward pass; inference writes the sigmoid output to ``out`` (float32
-        [B, n_out padded], row stride n_out padded) or to the workspace."""
+        [B, n_out padded], row stride n_out padded) or to the workspace. ``packed``: the
+        workspace already holds the standardised inputs."""
         B = ws.batch
         L = len(self.dims)
-        _lib.call("lbl_pack_inputs_bf16", ws.raw.data_ptr(), B, self.n_in, self.mean.data_ptr(),
-                  self.inv_std.data_ptr(), ws.x[0].data_ptr(), self.dims[0][0],
-                  ws.xt[0].data_ptr() if train else 0, B, stream)
-        self.launches += 1
+        if not packed:
+            _lib.call("lbl_pack_inputs_bf16", ws.raw.data_ptr(), B, self.n_in, self.mean.data_ptr(),
+                      self.inv_std.data_ptr(), ws.x[0].data_ptr(), self.dims[0][0],
+                      ws.xt[0].data_ptr() if train else 0, B, stream)
+            self.launches += 1
         for li, (k, n) in enumerate(self.dims):
             ep = _lib.GemmEpilogue()
             ep.bias = self.b[li].data_ptr()
@@ -407,14 +409,22 @@ class MLP:
         ws.target.copy_(target)
         return self._train_staged(ws, lr, check)
 
-    def _train_staged(self, ws: _Workspace, lr: Optional[float], check: bool = False):
-        """:meth:`train_step` on the batch already in ``ws.raw`` and ``ws.target``."""
+    def _train_staged(self, ws: _Workspace, lr: Optional[float], check: bool = False, samples=None):
+        """:meth:`train_step` on the batch already in ``ws.raw`` and ``ws.target``, or on the
+        samples (features, targets, indices)."""
         torch = self.torch
         B = ws.batch
         stream = torch.cuda.current_stream().cuda_stream
         self.launches = 0
-        ws.loss.zero_()
-        self._forward(ws, stream, True)
+        if samples is None:
+            ws.loss.zero_()
+        else:
+            x, y, idx = samples
+            _lib.call("lbl_stage_batch", x.data_ptr(), y.data_ptr(), idx.data_ptr(), x.shape[0], B, self.n_in,
+                      self.n_out, self.mean.data_ptr(), self.inv_std.data_ptr(), ws.x[0].data_ptr(), self.dims[0][0],
+                      ws.xt[0].data_ptr(), B, ws.target.data_ptr(), ws.loss.data_ptr(), stream)
+            self.launches += 1
+        self._forward(ws, stream, True, packed=samples is not None)
         self._backward(ws, stream)
         if self.world > 1:
             from . import shard
@@ -697,6 +707,8 @@ class Trainer:
         if self.x.shape[1:] != (net.n_in,) or self.y.shape[1:] != (net.n_out,):
             return net.train_step(self.x[idx], self.y[idx], lr=lr_at(cfg, net.step))
         ws = net.workspace(cfg.batch, True)          # the batch is gathered where the step reads it
+        if self.x.is_contiguous() and self.y.is_contiguous() and self.x.shape[0] == self.y.shape[0]:
+            return net._train_staged(ws, lr_at(cfg, net.step), samples=(self.x, self.y, idx))
         torch.index_select(self.x.detach(), 0, idx, out=ws.raw)
         torch.index_select(self.y.detach(), 0, idx, out=ws.target)
         return net._train_staged(ws, lr_at(cfg, net.step))

@@ -213,3 +213,29 @@ def test_gemm_pair_equals_single(cuda, shapes):
         assert torch.equal(x, y) and x.float().abs().sum() > 0
     want = (ab[1][0].float() @ ab[1][1].float().T)                      # the split sums are the product
     assert torch.allclose(outs[1][2].sum(0), want, rtol=1e-4, atol=1e-4 * shapes[1][2] ** 0.5)
+
+
+# remainders of the 32-row and 8-row splits, vector and scalar rows, several column blocks
+@pytest.mark.parametrize("rows,n_in,ld,n_out", [(1, 1, 128, 1), (33, 61, 128, 2000), (128, 130, 256, 301), (45, 64, 64, 8)])
+def test_stage_batch_equals_gather_and_pack(cuda, rows, n_in, ld, n_out):
+    g = torch.Generator(device="cuda").manual_seed(rows + n_in)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    n = 2 * rows + 5
+    feat, targ, mean, inv = rnd(n, n_in), rnd(n, n_out), rnd(n_in), rnd(n_in).abs() + 0.1
+    idx = torch.randperm(n, generator=torch.Generator().manual_seed(1)).cuda()[:rows]
+    bf = lambda *s: torch.full(s, 7.0, dtype=torch.bfloat16, device="cuda")
+    x, xt, x0, xt0 = bf(rows, ld), bf(ld, rows), bf(rows, ld), bf(ld, rows)
+    target = torch.full((rows, n_out), 7.0, device="cuda")
+    loss = torch.ones(1, dtype=torch.float64, device="cuda")
+    stage = lambda i: _lib.call("lbl_stage_batch", feat.data_ptr(), targ.data_ptr(), i.data_ptr(), n, rows, n_in, n_out,
+                                mean.data_ptr(), inv.data_ptr(), x.data_ptr(), ld, xt.data_ptr(), rows,
+                                target.data_ptr(), loss.data_ptr(), _stream())
+    stage(idx)
+    raw = feat[idx].contiguous()
+    _lib.call("lbl_pack_inputs_bf16", raw.data_ptr(), rows, n_in, mean.data_ptr(), inv.data_ptr(), x0.data_ptr(), ld,
+              xt0.data_ptr(), rows, _stream())
+    assert torch.equal(x, x0) and torch.equal(xt, xt0) and torch.equal(target, targ[idx]) and loss.item() == 0.0
+    out = idx.clone()
+    out[-1] = n                                       # not a sample: read nowhere, NaN in the batch
+    stage(out)
+    assert target[-1].isnan().all() and x[-1, :n_in].isnan().all() and torch.equal(target[:-1], targ[idx[:-1]])
