@@ -19,8 +19,9 @@ struct CellGeom {
 
 // A quarter of a chunk per cell: far cells (beyond four half-widths) then have |zeta| / |D| of
 // about 1/13. No cells where no line can be that far, for chunks shorter than two cells, or
-// for a grid of few chunks (each cell serves them all). The rule looks at the grid alone, so
-// a shard or a batch of profiles takes the same cells as the full job.
+// for a grid of few chunks (each cell serves them all). The rule looks at the grid alone and
+// split_lines at what lies inside the tile's window, so a shard takes the same cells as the
+// full job, bit for bit.
 static inline CellGeom cell_geometry(long long n_nu, int tile_samples, double step, double cutoff, int chunk_max) {
   const long long nch = (tile_samples + chunk_max - 1) / chunk_max;
   const long long n_c = tile_samples / nch;
@@ -66,8 +67,8 @@ struct LineSplit {
 };
 
 // Splits the lines rng of the tile [t0, t1) for the chunk at c0 of half-width H1 into n_use cells
-// (sh.use) that lie beyond four half-widths, inside the window and within their series'
-// radius with every line, and n_direct other lines in n_dir stretches. All threads of the CTA
+// (sh.use) that lie, with every line, beyond four half-widths, inside the window and within
+// their series' radius, and n_direct other lines in n_dir stretches. All threads of the CTA
 // call it. False: no cells considered, the lines are rng itself. REC: floats per record, GMAX:
 // the slot of g_max.
 template <int T, int REC, int GMAX>
@@ -100,15 +101,18 @@ __device__ __forceinline__ bool split_lines(LineSplit<T>& sh, const CellGeom& cg
           if (len > 0) {
             const float4 m = *reinterpret_cast<const float4*>(rec_row + (long long)q * REC + REC - 4);
             const float g_max = rec_row[(long long)q * REC + GMAX];
-            if (m.w == 0.f) len = 0;                       // only inactive lines
             const float pc = (float)((long long)q * cg.wp - cg.off - c0) + half;
+            // the cell itself inside the window, so that its choice cannot depend on lines
+            // beyond it, which a job of this tile's lines only does not hold
+            const bool inside = (double)(pc - half) >= wl && (double)(pc + half) <= wr && i0 == a && len == b - a;
+            if (inside && m.w == 0.f) len = 0;             // only inactive lines
             const float lo = pc + m.x, hi = pc + m.y;
             // all lines beyond four half-widths on one side, inside the window, in the far-wing
             // regime at the nearest node and well inside the series' radius
             const float gap = fmaxf(lo - (C1 + H1), (C1 - H1) - hi);
             const float z = fmaxf(fabsf(m.x), fabsf(m.y)) + g_max, D = fabsf(pc - C1) - H1;
-            use = m.w >= (float)CELL_MIN && i0 == a && len == b - a && gap > 3.f * H1 + 2.f && (double)lo >= wl &&
-                  (double)hi <= wr && m.z * gap >= 50.f && z <= CELL_RATIO * D;
+            use = inside && m.w >= (float)CELL_MIN && gap > 3.f * H1 + 2.f && (double)lo >= wl && (double)hi <= wr &&
+                  m.z * gap >= 50.f && z <= CELL_RATIO * D;
           }
         }
         const unsigned bu = __ballot_sync(0xffffffffu, use), bd = __ballot_sync(0xffffffffu, len > 0 && !use);
