@@ -11,6 +11,7 @@ constexpr float CELL_RATIO = 1.0f / 6.5f;
 constexpr int CELL_MIN = 4;                    // fewer lines are cheaper one by one
 constexpr int CELL_MIN_CHUNKS = 16;            // fewer chunks on the grid: no cells
 constexpr int CELL_MIN_PTS = 64;               // smallest cell (bounds the records to 1 byte per point and row)
+constexpr int LINE_CELLS = 512;                // most cells of a tile's window (more: every line by itself)
 
 struct CellGeom {
   int wp, n;            // points per cell, cells (0: none)
@@ -18,10 +19,13 @@ struct CellGeom {
 };
 
 // A quarter of a chunk per cell: far cells (beyond four half-widths) then have |zeta| / |D| of
-// about 1/13. No cells where no line can be that far, for chunks shorter than two cells, or
-// for a grid of few chunks (each cell serves them all). The rule looks at the grid alone and
-// split_lines at what lies inside the tile's window, so a shard takes the same cells as the
-// full job, bit for bit.
+// about 1/13. No cells where no line can be that far, for chunks shorter than two cells, for a
+// grid of few chunks (each cell serves them all), or where a full tile's window holds more
+// cells than split_lines takes, since their moments would be formed and never used (25 cm^-1
+// cut-off: tiles below 0.4 cm^-1 at 0.001 cm^-1; 2 cm^-1 tiles at 0.0002 cm^-1 and finer, the
+// Jacobian's shorter chunks at 0.0004). The rule looks at the grid alone and split_lines at
+// what lies inside the tile's window, so a shard takes the same cells as the full job, bit for
+// bit.
 static inline CellGeom cell_geometry(long long n_nu, int tile_samples, double step, double cutoff, int chunk_max) {
   const long long nch = (tile_samples + chunk_max - 1) / chunk_max;
   const long long n_c = tile_samples / nch;
@@ -31,6 +35,8 @@ static inline CellGeom cell_geometry(long long n_nu, int tile_samples, double st
       (n_nu + tile_samples - 1) / tile_samples * nch < CELL_MIN_CHUNKS)
     return g;
   g.wp = (int)(n_c / 4 > CELL_MIN_PTS ? n_c / 4 : CELL_MIN_PTS);
+  const long long tile = tile_samples < n_nu ? tile_samples : n_nu;
+  if ((tile + 2 * (long long)reach) / g.wp + 6 > LINE_CELLS) return CellGeom{0, 0, 0};   // qe - qa of split_lines
   g.off = ((long long)reach / g.wp + 2) * g.wp;
   const long long n = (n_nu + 2 * g.off + g.wp - 1) / g.wp;
   if (n > 0x3fffffff) return CellGeom{0, 0, 0};
@@ -56,8 +62,6 @@ static __global__ void cell_bounds_kernel(const LineIn* __restrict__ lines, cons
 // four floats are e_min, e_max (the lines' extent about the cell's centre, points), a_min and
 // the number of active lines (-1: a line too broad or of negative width).
 static inline long long cell_head(const CellGeom& g) { return ((long long)g.n + 1 + 3) / 4 * 4; }
-
-constexpr int LINE_CELLS = 512;   // most cells of a tile's window (more: every line by itself)
 
 template <int T>
 struct LineSplit {
