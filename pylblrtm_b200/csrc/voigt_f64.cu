@@ -94,16 +94,17 @@ __device__ __forceinline__ double wing_f64(double x, double y2) {
 }
 
 // Re w at one point, any z: the series cut after 7, 13 or 22 terms, Weideman's 48-term
-// approximation inside |z|^2 < CORE_F64_Z2. One of the forms per warp outside the core (the
-// longest that a lane needs), so at most two run.
+// approximation inside |z|^2 < CORE_F64_Z2. All 32 lanes of a warp call it together: outside
+// the core the warp takes one form, the longest that one of its lanes needs, so at most two
+// run and the choice depends on the lanes' arguments alone.
 __device__ __forceinline__ double voigt_re_f64(double x, double y) {
   const double y2 = y * y, z2 = fma(x, x, y2);
   const bool up = y >= 0.0;
-  const unsigned m = __activemask();
-  if (!__any_sync(m, !(up && z2 >= ASYM_Z2))) return INV_SQRT_PI * y * wing_f64<7>(x, y2);
+  if (!__any_sync(0xffffffffu, !(up && z2 >= ASYM_Z2))) return INV_SQRT_PI * y * wing_f64<7>(x, y2);
+  const bool s22 = __any_sync(0xffffffffu, up && z2 >= CORE_F64_Z2 && z2 < ASYM13_Z2);
   if (up && z2 >= CORE_F64_Z2) {
     const double r = rcp_f64(z2);
-    return __any_sync(__activemask(), z2 < ASYM13_Z2) ? re_w_series<22>(x * r, -y * r) : re_w_series<13>(x * r, -y * r);
+    return s22 ? re_w_series<22>(x * r, -y * r) : re_w_series<13>(x * r, -y * r);
   }
   return core_f64(x, y);
 }
@@ -222,11 +223,12 @@ tau_f64_kernel(const LineF64* __restrict__ prep, int n_lines, const int2* __rest
       const double nu = grid_nu(nu_min, step, c0 + p);
       double acc = 0.0;
       np = 0;
-      for (int li = rng.x + tid; li < rng.y; li += D_THREADS) {
+      for (int base = rng.x; base < rng.y; base += D_THREADS) {   // whole warps, absent lines as zeros
         LineF64 L;
-        if (!load(li, L)) continue;
-        ++np;
-        acc = fma(L.amp, voigt_re_f64((nu - L.nuc) * L.inv_ad, L.y), acc);
+        const bool on = load(base + tid, L);
+        np += on;
+        const double v = voigt_re_f64(on ? (nu - L.nuc) * L.inv_ad : 100.0, on ? L.y : 1.0);
+        acc = fma(on ? L.amp : 0.0, v, acc);
       }
       for (int o = 16; o > 0; o >>= 1) acc += shfl_xor_f64(acc, o);
       if (lane == 0) s_part[warp][0] = acc;
