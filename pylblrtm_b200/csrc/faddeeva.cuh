@@ -250,9 +250,10 @@ LBL_HD double weideman_re_f32(double x, double y) { return weideman_re<LBL_WEIDE
 // The same by complex Horner, for rarely taken paths of kernels at their register limit.
 LBL_HD double weideman_re_f32_compact(double x, double y) { return weideman_re<LBL_WEIDEMAN28_N, true>(x, y); }
 
-// Re w inside |z|^2 < 49 for the float64 engine: the 48-term set (against scipy.special.wofz
-// within 5e-12 of Re w for y >= 1e-3 and 5e-11 for y >= 1e-4; the Maclaurin and Taylor
-// branches of faddeeva() above reach 2e-8 and 2e-7 there).
+// Re w by the 48-term set, as the float64 engine takes it in the core (re_w_f64_core below):
+// against scipy.special.wofz within 5e-12 of Re w for y >= 1e-3 and 5e-11 for y >= 1e-4, growing
+// as 1/y below (2e-9 at 1e-6, 2e-7 at 1e-8); the Maclaurin and Taylor branches of faddeeva()
+// above reach 2e-8 and 2e-7 at y = 1e-3 and 1e-4, 2e-3 at 1e-8.
 LBL_HD double weideman_re_f64(double x, double y) { return weideman_re<LBL_WEIDEMAN48_N>(x, y); }
 
 // Re w by N terms of the asymptotic series (i/sqrt(pi)) sum (2k-1)!!/2^k z^-(2k+1), complex
@@ -273,6 +274,108 @@ LBL_HD double re_w_series(double zr, double zi) {
     pr = t;
   }
   return -INV_SQRT_PI * fma(zr, pi, zi * pr);
+}
+
+// ---- Re w of the float64 engine, by |z|^2; y >= 0 unless said otherwise.
+constexpr double ASYM_Z2 = 400.0;    // seven asymptotic terms: first omitted term <= 2e-16 of Re w
+constexpr double ASYM13_Z2 = 100.0;  // thirteen terms: <= 3e-16
+constexpr double CORE_F64_Z2 = 49.0; // twenty-two terms: <= 3e-14
+constexpr double ASYM4_Z2 = 5.0e3;   // four terms: <= 1e-16
+constexpr double ASYM2_Z2 = 4.5e5;   // two terms: <= 2e-16
+
+// 1/v for normal v > 0. On the device from rcp.approx.ftz.f64, whose result r carries the top 20
+// bits of the mantissa: with e = 1 - v r, 1/v = r / (1 - e) = r (1 + e + e^2 + ...), cut after
+// e^2 (omitted: e^3 ~ 2^-60), so what is left is the rounding of the last fma, about 2^-53.
+LBL_HD double rcp_f64(double v) {
+#ifdef __CUDA_ARCH__
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(v));
+  const double e = fma(-v, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+#else
+  return 1.0 / v;
+#endif
+}
+
+// sqrt(pi) Re w / y = r (1 + sum_k r^k A_k(q)), r = 1/|z|^2, q = y^2 r, cut after N terms
+// (A_k as in re_w_asym8 below).
+template <int N>
+LBL_HD double wing_f64(double x, double y2) {
+  const double r = rcp_f64(fma(x, x, y2)), q = y2 * r;
+  double s = 0.0;
+  if constexpr (N >= 7) {
+    const double a7 = fma(fma(fma(fma(fma(fma(fma(-17297280.0, q, 64864800.0), q, -97297200.0), q, 74324250.0),
+                                      q, -30405375.0), q, 6385128.75), q, -591215.625), q, 15836.1328125);
+    const double a6 = fma(fma(fma(fma(fma(fma(665280.0, q, -2162160.0), q, 2702700.0), q, -1621620.0), q, 472972.5),
+                              q, -59121.5625), q, 2111.484375);
+    const double a5 = fma(fma(fma(fma(fma(-30240.0, q, 83160.0), q, -83160.0), q, 36382.5), q, -6496.875), q, 324.84375);
+    s = fma(fma(a7, r, a6), r, a5);
+  }
+  if constexpr (N >= 4) {
+    const double a4 = fma(fma(fma(fma(1680.0, q, -3780.0), q, 2835.0), q, -787.5), q, 59.0625);
+    const double a3 = fma(fma(fma(-120.0, q, 210.0), q, -105.0), q, 13.125);
+    s = N >= 7 ? fma(fma(s, r, a4), r, a3) : fma(a4, r, a3);
+  }
+  const double a2 = fma(fma(12.0, q, -15.0), q, 3.75);
+  s = N >= 4 ? fma(s, r, a2) : a2;
+  s = fma(s, r, fma(-2.0, q, 1.5));
+  return fma(s * r, r, r);
+}
+
+// The real part that the asymptotic series and the quadrature below leave out on and near the
+// real axis, exp(y^2 - x^2) cos(2xy): all of Re w at y = 0. The cosine to second order: where the two
+// are used (q = 2xy), q^4 / 24 of it stays below 1e-14 of Re w.
+LBL_HD double axis_term_f64(double x, double y) { return exp(y * y - x * x) * fma(-2.0 * (x * y), x * y, 1.0); }
+
+// Whether the seven-term series is Re w to double precision. Below y = 1e-140 the axis term
+// (1e-174 at |z|^2 = 400) shows until it underflows.
+LBL_HD bool wing_only_f64(double y, double z2) { return z2 >= ASYM_Z2 && (y >= 1e-140 || (y >= 0.0 && z2 >= 760.0)); }
+
+// Re w for |z|^2 >= CORE_F64_Z2: 22 terms (s22, needed below ASYM13_Z2) or 13, and the axis term
+// for widths so small that it reaches 1e-16 of y / (sqrt(pi) |z|^2).
+LBL_HD double re_w_f64_series(double x, double y, bool s22) {
+  const double z2 = fma(x, x, y * y), r = rcp_f64(z2);
+  const double v = s22 ? re_w_series<22>(x * r, -y * r) : re_w_series<13>(x * r, -y * r);
+  return y < (z2 < ASYM13_Z2 ? 5e-4 : z2 < ASYM_Z2 ? 1e-20 : 1e-140) ? v + axis_term_f64(x, y) : v;
+}
+
+// Re w by 16-point Gauss-Hermite quadrature of (y/pi) int exp(-t^2) / ((x - t)^2 + y^2) dt (the
+// 16th convergent of the Laplace continued fraction), the nodes in pairs +-t_k, and the axis term.
+// Every term carries the factor y: for |z|^2 >= HERMITE_Z2 within 3e-11 of Re w however small y
+// is, 5e-12 from 33, 6e-13 from 36 and 2e-14 from 42 on.
+constexpr double HERMITE_Z2 = 28.409;
+LBL_HD double re_w_hermite(double x, double y) {
+  const double t2[8] = {LBL_HERMITE16_T2}, w[8] = {LBL_HERMITE16_W};
+  const double x2 = x * x, y2 = y * y, z2 = x2 + y2;
+  double s = 0.0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const double d = x2 - t2[k];
+    s = fma(w[k] * (z2 + t2[k]), rcp_f64(fma(d, d, y2 * fma(2.0, x2 + t2[k], y2))), s);
+  }
+  return fma(y, s, axis_term_f64(x, y));
+}
+
+// Re w for |z|^2 < CORE_F64_Z2. Weideman's 48 terms are uniform to 2e-16 of w(0), so their error
+// relative to Re w ~ y / (sqrt(pi) |z|^2) grows as 1/y; the quadrature takes over where it is the better one.
+LBL_HD double re_w_f64_core(double x, double y) {
+  const double z2 = fma(x, x, y * y);
+  if (z2 >= HERMITE_Z2 && y < (z2 >= 42.0 ? 0.5 : z2 >= 36.0 ? 0.01 : z2 >= 33.0 ? 1e-3 : 3e-4)) return re_w_hermite(x, y);
+  return weideman_upper_n<LBL_WEIDEMAN48_N>(x, y).re;
+}
+
+// Re w(x - i ay) from v = Re w(x + i ay).
+LBL_HD double re_w_f64_lower(double x, double ay, double v) {
+  return 2.0 * exp(ay * ay - x * x) * cos(2.0 * x * ay) - v;
+}
+
+// Re w for any z, one argument at a time (the kernel takes the series' length warp by warp).
+LBL_HD double re_w_f64_any(double x, double y) {
+  const double ay = fabs(y), z2 = fma(x, x, ay * ay);
+  const double v = wing_only_f64(ay, z2)   ? INV_SQRT_PI * ay * wing_f64<7>(x, ay * ay)
+                   : z2 >= CORE_F64_Z2 ? re_w_f64_series(x, ay, z2 < ASYM13_Z2)
+                                       : re_w_f64_core(x, ay);
+  return y >= 0.0 ? v : re_w_f64_lower(x, ay, v);
 }
 
 // |z|^2 below which the engine evaluates Re w in double precision (Weideman's

@@ -23,6 +23,11 @@ int lbl_host_weideman_re(const double* x, const double* y, long long n, int term
   return 0;
 }
 
+// Re w as the float64 engine computes it, any y.
+void lbl_host_re_w_f64(const double* x, const double* y, long long n, double* re) {
+  for (long long i = 0; i < n; ++i) re[i] = lbl::re_w_f64_any(x[i], y[i]);
+}
+
 // Re w by the float64 engine's asymptotic series (terms = 13 or 22), y >= 0.
 int lbl_host_series_re(const double* x, const double* y, long long n, int terms, double* re) {
   if (terms != 13 && terms != 22) return -1;

@@ -16,19 +16,22 @@
 //            chunk, again one per thread; those not far of the sub-chunk go to a list;
 //   level 3  32-point segments, one per warp: far lines of the list at 16 nodes, one per
 //            lane; the remaining lines directly, one point per lane.
-// A far line also needs |z|^2 >= ASYM_Z2 at its nearest node, so every node value is the
-// asymptotic series in its real-part form with one reciprocal; what fails that test is
-// summed directly at each point (longer series, Weideman's approximation in the core). Every
+// A far line also needs |z|^2 >= ASYM_Z2 at its nearest node and a width that is not
+// negative, so every node value is the asymptotic series in its real-part form with one
+// reciprocal; what fails that test is summed directly at each point (faddeeva.cuh has the
+// forms by distance). Every
 // sum is formed in a fixed order (no floating-point atomics), so results are bit-reproducible.
 //
 // Bound by float64 issue and latency (two CTAs per SM at 128 registers): about 240 node
 // values and 20 direct values per point and layer at 105 lines per cm^-1, 0.001 cm^-1 steps
 // and a 25 cm^-1 cut-off, where evaluating every line at every point by the Gautschi method
 // takes 5,500. Kernel times on B200, before (every line at every point) and now: 20 cm^-1 of
-// a 200,000-line list at 60 layers 91.9 -> 0.84 ms, 20 cm^-1 of a 2,000-line band at 20
-// layers 14.6 -> 0.135 ms. Chunks of 512, 1,024 and 2,048 points measure the same on the
-// former (0.84, 0.86, 0.9 ms) and 0.135, 0.16, 0.3 ms on the latter (too few CTAs); D_FAR of
-// 5 or 8 instead of 6 changes less than 5 %.
+// a 200,000-line list at 60 layers 91.9 -> 0.92 ms, 20 cm^-1 of a 2,000-line band at 20
+// layers 14.6 -> 0.147 ms (0.84 and 0.142 without the quadrature next to the real axis, which
+// keeps the accuracy of the former method for lines of small width). Chunks of 512, 1,024 and
+// 2,048 points measure the same on the former (0.84, 0.86, 0.9 ms without the quadrature) and
+// 0.135, 0.16, 0.3 ms on the latter (too few CTAs); D_FAR of 5 or 8 instead of 6 changes less
+// than 5 %.
 #include <math.h>
 
 #include "cheb_tables.h"
@@ -48,65 +51,27 @@ constexpr int D_LIST = 768;        // listed lines per sub-chunk between two pas
 constexpr int D_FEW = 16;          // a chunk of at most D_K points takes every line at every point
 constexpr double D_FAR = 6.0;
 
-constexpr double ASYM_Z2 = 400.0;  // seven asymptotic terms: first omitted term <= 2e-16 of Re w
-constexpr double ASYM13_Z2 = 100.0;  // thirteen terms: <= 3e-16
-constexpr double CORE_F64_Z2 = 49.0; // twenty-two terms: <= 4e-16 (and exp(-x^2) below 1e-14 of Re w for y >= 1e-5)
-constexpr double ASYM4_Z2 = 5.0e3; // four terms: <= 1e-16
-constexpr double ASYM2_Z2 = 4.5e5; // two terms: <= 2e-16
-
 static __constant__ double c_ddct16[D_K * D_K] = {LBL_DCT16};
 // node k (fraction of the half-width): cos((2k+1) pi/32), row 1 of the DCT table
 #define D_NODE(k) c_ddct16[D_K + (k)]
 
-// 1/v for normal v > 0: the hardware's ~20-bit estimate and one cubic step (error 2^-60).
-__device__ __forceinline__ double rcp_f64(double v) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(v));
-  const double e = fma(-v, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
+// The forms of the core and the reflection below the axis, out of line (registers, code size).
+static __device__ __noinline__ double core_f64(double x, double y) { return re_w_f64_core(x, y); }
+static __device__ __noinline__ double lower_f64(double x, double ay, double v) { return re_w_f64_lower(x, ay, v); }
 
-// sqrt(pi) Re w / y = r (1 + sum_k r^k A_k(q)), r = 1/|z|^2, q = y^2 r, cut after N terms
-// (A_k as in re_w_asym8 of faddeeva.cuh).
-static __device__ __noinline__ double core_f64(double x, double y) { return weideman_re_f64(x, y); }
-
-template <int N>
-__device__ __forceinline__ double wing_f64(double x, double y2) {
-  const double r = rcp_f64(fma(x, x, y2)), q = y2 * r;
-  double s = 0.0;
-  if constexpr (N >= 7) {
-    const double a7 = fma(fma(fma(fma(fma(fma(fma(-17297280.0, q, 64864800.0), q, -97297200.0), q, 74324250.0),
-                                      q, -30405375.0), q, 6385128.75), q, -591215.625), q, 15836.1328125);
-    const double a6 = fma(fma(fma(fma(fma(fma(665280.0, q, -2162160.0), q, 2702700.0), q, -1621620.0), q, 472972.5),
-                              q, -59121.5625), q, 2111.484375);
-    const double a5 = fma(fma(fma(fma(fma(-30240.0, q, 83160.0), q, -83160.0), q, 36382.5), q, -6496.875), q, 324.84375);
-    s = fma(fma(a7, r, a6), r, a5);
-  }
-  if constexpr (N >= 4) {
-    const double a4 = fma(fma(fma(fma(1680.0, q, -3780.0), q, 2835.0), q, -787.5), q, 59.0625);
-    const double a3 = fma(fma(fma(-120.0, q, 210.0), q, -105.0), q, 13.125);
-    s = N >= 7 ? fma(fma(s, r, a4), r, a3) : fma(a4, r, a3);
-  }
-  const double a2 = fma(fma(12.0, q, -15.0), q, 3.75);
-  s = N >= 4 ? fma(s, r, a2) : a2;
-  s = fma(s, r, fma(-2.0, q, 1.5));
-  return fma(s * r, r, r);
-}
-
-// Re w at one point, any z: the series cut after 7, 13 or 22 terms, Weideman's 48-term
-// approximation inside |z|^2 < CORE_F64_Z2. All 32 lanes of a warp call it together: outside
-// the core the warp takes one form, the longest that one of its lanes needs, so at most two
-// run and the choice depends on the lanes' arguments alone.
+// Re w at one point, any z. All 32 lanes of a warp call it together: outside the core the warp
+// takes one form, the longest that one of its lanes needs, so at most two run and the choice
+// depends on the lanes' arguments alone.
 __device__ __forceinline__ double voigt_re_f64(double x, double y) {
-  const double y2 = y * y, z2 = fma(x, x, y2);
-  const bool up = y >= 0.0;
-  if (!__any_sync(0xffffffffu, !(up && z2 >= ASYM_Z2))) return INV_SQRT_PI * y * wing_f64<7>(x, y2);
-  const bool s22 = __any_sync(0xffffffffu, up && z2 >= CORE_F64_Z2 && z2 < ASYM13_Z2);
-  if (up && z2 >= CORE_F64_Z2) {
-    const double r = rcp_f64(z2);
-    return s22 ? re_w_series<22>(x * r, -y * r) : re_w_series<13>(x * r, -y * r);
+  const double ay = fabs(y), y2 = ay * ay, z2 = fma(x, x, y2);
+  double v;
+  if (!__any_sync(0xffffffffu, !wing_only_f64(ay, z2))) {
+    v = INV_SQRT_PI * ay * wing_f64<7>(x, y2);
+  } else {
+    const bool s22 = __any_sync(0xffffffffu, z2 >= CORE_F64_Z2 && z2 < ASYM13_Z2);
+    v = z2 >= CORE_F64_Z2 ? re_w_f64_series(x, ay, s22) : core_f64(x, ay);
   }
-  return core_f64(x, y);
+  return y >= 0.0 ? v : lower_f64(x, ay, v);
 }
 
 template <int N>
@@ -130,7 +95,7 @@ __device__ __forceinline__ bool far_nodes_add(double (&f)[D_K], const LineF64& L
   const double d = __dsub_rn(s.c, L.nuc), ad = fabs(d);
   const double xm = __dmul_rn(__dsub_rn(ad, s.h), L.inv_ad);         // |x| at the interval's near end
   const double y2 = __dmul_rn(L.y, L.y), zm = __dadd_rn(__dmul_rn(xm, xm), y2);
-  if (!(ad > __dmul_rn(D_FAR, s.h) && zm >= ASYM_Z2 && L.y >= 0.0)) return false;
+  if (!(ad > __dmul_rn(D_FAR, s.h) && wing_only_f64(L.y, zm))) return false;
   if (add) {
     const double xc = d * L.inv_ad, ha = s.h * L.inv_ad, af = L.amp * L.y * INV_SQRT_PI;
     if (zm >= ASYM2_Z2) nodes_add_n<2>(f, xc, ha, y2, af);
