@@ -158,12 +158,11 @@ __device__ __forceinline__ float reduce_nodes16(const float (&f)[16], int lane) 
   return v + __shfl_xor_sync(full, v, 1);
 }
 
-// Adds the lanes' float node sums into the warp's float64 sums and clears them; every lane of
-// the warp calls it. K = 16 or 8. The sums are formed in float64 by a transposed reduction
-// (32 or 18 shuffles where a reduction per node took 160 or 80; the flush had been half of the
-// level-1 kernel's instructions once most of its lines went through cells).
+// The same in float64 for K = 16 or 8 float sums, which are cleared: lanes (32 / K) j and up hold
+// the total of node j (32 or 18 shuffles where a reduction per node took 160 or 80; the flush had
+// been half of the level-1 kernel's instructions once most of its lines went through cells).
 template <int K>
-__device__ __forceinline__ void flush_nodes(float (&f)[K], double* row, int lane) {
+__device__ __forceinline__ double reduce_nodes_f64(float (&f)[K], int lane) {
   static_assert(K == 16 || K == 8, "node counts");
   constexpr unsigned full = 0xffffffffu;
   double g[K / 2];
@@ -178,12 +177,19 @@ __device__ __forceinline__ void flush_nodes(float (&f)[K], double* row, int lane
   double v;
   if constexpr (K == 16) v = (b1 ? g[1] : g[0]) + __shfl_xor_sync(full, b1 ? g[0] : g[1], 2);
   else v = g[0] + __shfl_xor_sync(full, g[0], 2);
-  v += __shfl_xor_sync(full, v, 1);
-  constexpr int per = 32 / K;                                  // lanes per node
-  if (lane % per == 0) row[lane / per] += v;
 #pragma unroll
   for (int k = 0; k < K; ++k) f[k] = 0.f;
-  __syncwarp(full);
+  return v + __shfl_xor_sync(full, v, 1);
+}
+
+// Adds the lanes' float node sums into the warp's float64 sums and clears them; every lane of
+// the warp calls it.
+template <int K>
+__device__ __forceinline__ void flush_nodes(float (&f)[K], double* row, int lane) {
+  const double v = reduce_nodes_f64(f, lane);
+  constexpr int per = 32 / K;                                  // lanes per node
+  if (lane % per == 0) row[lane / per] += v;
+  __syncwarp(0xffffffffu);
 }
 
 static __device__ __noinline__ float re_w_f32_mid(float x, float y, float y2, float z2) {

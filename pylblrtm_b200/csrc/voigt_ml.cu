@@ -144,6 +144,7 @@ __device__ __forceinline__ void clenshaw_points(const float (&c)[ML_K], const f3
 // ~ 1e-8 of the cell's field; nothing cancels that the lines' own rounding would not show.
 constexpr int CELL_M = 11;                     // moments k = 1 .. 11
 constexpr int CELL_F = 16;                     // floats per record: moments, g_max, e_min, e_max, a_min, lines
+constexpr int MF_FLUSH = 32;                   // lines or cells a thread sums in float before the double sums
 // One warp per (cell, row).
 __global__ void __launch_bounds__(256)
 line_moments_kernel(const LineF32* __restrict__ prep, int n_lines, const int* __restrict__ idx, CellGeom cg,
@@ -163,11 +164,10 @@ line_moments_kernel(const LineF32* __restrict__ prep, int n_lines, const int* __
 #pragma unroll
   for (int k = 0; k < ML_K; ++k) m[k] = 0.f;
   float e_min = 3.0e38f, e_max = -3.0e38f, a_min = 3.0e38f, g_max = 0.f;
-  int cnt = 0;
+  int cnt = 0, rounds = 0;
   bool ok = true;
-  for (int li = i0 + lane; li < i1; li += 32) {
-    const LineF32 L = lp[li];
-    if (!(L.nuc == L.nuc)) continue;                   // inactive
+  double v = 0.0;                                      // lanes 2j, 2j + 1: moment j + 1
+  auto add = [&](const LineF32& L) {
     ++cnt;
     const float inv_a = 1.0f / L.a;
     const float e = (float)(L.j0 - jb) - half + L.b * inv_a, g = L.y * inv_a;
@@ -189,8 +189,18 @@ line_moments_kernel(const LineF32* __restrict__ prep, int n_lines, const int* __
       R = Rn;
       J = Jn;
     }
+  };
+  for (int base = i0; base < i1; base += 32) {
+    const int li = base + lane;
+    if (li < i1) {
+      const LineF32 L = lp[li];
+      if (L.nuc == L.nuc) add(L);                      // not an inactive one
+    }
+    if (++rounds == MF_FLUSH || base + 32 >= i1) {     // warp-uniform
+      rounds = 0;
+      v += reduce_nodes_f64(m, lane);
+    }
   }
-  const float v = reduce_nodes16(m, lane);        // lanes 2j, 2j + 1: moment j + 1
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1) {
     e_min = fminf(e_min, __shfl_xor_sync(0xffffffffu, e_min, o));
@@ -200,7 +210,7 @@ line_moments_kernel(const LineF32* __restrict__ prep, int n_lines, const int* __
   }
   cnt = __reduce_add_sync(0xffffffffu, cnt);
   ok = __all_sync(0xffffffffu, ok);
-  if (!(lane & 1) && (lane >> 1) < CELL_M) out[lane >> 1] = v;
+  if (!(lane & 1) && (lane >> 1) < CELL_M) out[lane >> 1] = (float)v;
   if (lane == 1) {
     out[CELL_M] = g_max;
     out[CELL_M + 1] = e_min;
@@ -221,10 +231,10 @@ line_moments_kernel(const LineF32* __restrict__ prep, int n_lines, const int* __
 // loads, so small CTAs, sixteen to an SM, cover each other's waits. Whole spectrum (200,000
 // lines, 60 layers, 950 tiles) on B200: every line by itself 1,764 us; with cells 1,209, with
 // the transposed flush 1,001, and with CTAs of 128 and 64 instead of 256 threads 688 and 610 us
-// (plus 125 us for the moments, which read the 384 MB of records once).
+// (plus 160 us for the moments, which read the 384 MB of records once; 125 with float32 sums
+// across the lanes, which put the error of far wings at 1.4 times the line-by-line error
+// instead of 1.15).
 constexpr int MF_THREADS = 64;                 // lines per round
-constexpr int MF_FLUSH = 32;                   // rounds summed in float before the double sums
-
 constexpr int MF_STAGES = 3;                   // rounds of line records in flight per thread
 
 // amp * Re w by the far-wing form (amp_far = amp y / sqrt(pi)), added to f (|z|^2 >= FAR_Z2, y >= 0).
@@ -293,7 +303,7 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
   __shared__ float s_coef[ML_K + ML_KF];
   __shared__ unsigned s_cnt[3];
   __shared__ LineSplit<MF_THREADS> s_split;
-  __shared__ float s_cell[MF_THREADS / 32][ML_KF];
+  __shared__ double s_cell[MF_THREADS / 32][ML_KF];
 
   const int row = blockIdx.y;
   const int tile = tile_first + (int)(blockIdx.x / chunks_per_tile), chunk = blockIdx.x % chunks_per_tile;
@@ -336,10 +346,17 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
     const int k = tid & (ML_KF - 1);
     const float xk = k < ML_KF / 2 ? H1 * c_node8[k] : -H1 * c_node8[ML_KF - 1 - k];
     const float half = 0.5f * (float)cg.wp;
+    double sum = 0.0;
     float f = 0.f;
     unsigned c = 0;
+    int rounds = 0;
 #pragma unroll 4
     for (int i = tid >> 3; i < n_use; i += MF_THREADS / 8) {
+      if (++rounds > MF_FLUSH) {
+        rounds = 1;
+        sum += (double)f;
+        f = 0.f;
+      }
       const int q = s_split.use[i];
       const float4* r4 = reinterpret_cast<const float4*>(rec_row + (long long)q * CELL_F);
       const float4 a = r4[0], b = r4[1], d = r4[2];
@@ -358,10 +375,11 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
       v = fmaf(v, t, a.x);
       f = fmaf(rD * rD, v, f);
     }
-    f += __shfl_xor_sync(0xffffffffu, f, 8);
-    f += __shfl_xor_sync(0xffffffffu, f, 16);
+    sum += (double)f;
+    sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 16);
     c = __reduce_add_sync(0xffffffffu, c);
-    if (lane < ML_KF) s_cell[warp][lane] = f;
+    if (lane < ML_KF) s_cell[warp][lane] = sum;
     if (lane == 0) atomicAdd(&s_cnt[2], c);
   }
 
@@ -429,7 +447,7 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
     double s = 0.0;
     for (int w = 0; w < MF_THREADS / 32; ++w) s += s_part[w][tid];
     if (cells && tid >= ML_K)
-      for (int w = 0; w < MF_THREADS / 32; ++w) s += (double)s_cell[w][tid - ML_K];
+      for (int w = 0; w < MF_THREADS / 32; ++w) s += s_cell[w][tid - ML_K];
     s_part[0][tid] = s;
   }
   __syncthreads();

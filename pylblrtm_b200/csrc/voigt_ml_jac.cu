@@ -326,12 +326,10 @@ jac_moments_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__
 #pragma unroll
     for (int k = 0; k < MJ_K; ++k) m[p][k] = 0.f;
   float e_min = 3.0e38f, e_max = -3.0e38f, a_min = 3.0e38f, g_max = 0.f;
-  int cnt = 0;
+  int cnt = 0, rounds = 0;
   bool ok = true;
-  for (int li = i0 + lane; li < i1; li += 32) {
-    const LineF32 L = lp[li];
-    if (!(L.nuc == L.nuc)) continue;               // inactive
-    const LineJac J = jp[li];
+  double v[3] = {0.0, 0.0, 0.0};                   // lanes 2j, 2j + 1: moment j + 1 of each sum
+  auto add = [&](const LineF32& L, const LineJac& J) {
     ++cnt;
     const float ia = 1.0f / L.a;
     const float e = (float)(L.j0 - jb) - s + L.b * ia, g = L.y * ia;
@@ -340,9 +338,7 @@ jac_moments_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__
     e_max = fmaxf(e_max, e);
     a_min = fminf(a_min, L.a);
     g_max = fmaxf(g_max, g);
-    const float zr = e * inv_s, zi = g * inv_s, k0 = float(INV_SQRT_PI);
-    const float w0 = k0 * L.amp, wu = k0 * J.jT_u, wx = k0 * J.jT_x, wy = k0 * J.jT_y;
-    const float vu = k0 * J.jv_u, vy = k0 * J.jv_y, vx = k0 * J.jv_x;
+    const float zr = e * inv_s, zi = g * inv_s;
     const float ia2 = ia * ia, c3 = inv_s * ia2, c4 = inv_s * inv_s * ia2;   // 1/(s a^2), 1/(s^2 a^2)
     // R, I: real and imaginary part of (zeta / s)^k; R1.. one, two and three powers before
     float R = zr, I = zi, R1 = 1.f, I1 = 0.f, R2 = 0.f, I2 = 0.f, R3 = 0.f, I3 = 0.f;
@@ -354,18 +350,28 @@ jac_moments_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__
       const float U = ia * fmaf(0.5f, iv3, iv);
       const float X = ia * fmaf(1.5f, fmaf(g, rv4, iv3), fmaf(g, rv2, iv));
       const float Y = ia2 * fmaf(1.5f, rv4, rv2), Z = ia2 * fmaf(1.5f, iv4, iv2);
-      m[0][k - 1] = fmaf(w0, U, m[0][k - 1]);
-      m[1][k - 1] = fmaf(wu, U, fmaf(wx, X, fmaf(-wy, Y, m[1][k - 1])));
-      m[2][k - 1] = fmaf(vu, U, fmaf(vy, Y, fmaf(vx, Z, m[2][k - 1])));
+      m[0][k - 1] = fmaf(L.amp, U, m[0][k - 1]);
+      m[1][k - 1] = fmaf(J.jT_u, U, fmaf(J.jT_x, X, fmaf(-J.jT_y, Y, m[1][k - 1])));
+      m[2][k - 1] = fmaf(J.jv_u, U, fmaf(J.jv_y, Y, fmaf(J.jv_x, Z, m[2][k - 1])));
       const float Rn = fmaf(R, zr, -I * zi), In = fmaf(R, zi, I * zr);
       R3 = R2; I3 = I2; R2 = R1; I2 = I1; R1 = R; I1 = I; R = Rn; I = In;
     }
+  };
+  for (int base = i0; base < i1; base += 32) {
+    const int li = base + lane;
+    if (li < i1) {
+      const LineF32 L = lp[li];
+      if (L.nuc == L.nuc) add(L, jp[li]);          // not an inactive one
+    }
+    if (++rounds == MJF_FLUSH || base + 32 >= i1) {   // warp-uniform
+      rounds = 0;
+#pragma unroll
+      for (int p = 0; p < 3; ++p) v[p] += reduce_nodes_f64(m[p], lane);
+    }
   }
 #pragma unroll
-  for (int p = 0; p < 3; ++p) {
-    const float v = reduce_nodes16(m[p], lane);    // lanes 2j, 2j + 1: moment j + 1
-    if (!(lane & 1) && (lane >> 1) < JC_M) out[p * (JC_M + 1) + (lane >> 1)] = v;
-  }
+  for (int p = 0; p < 3; ++p)
+    if (!(lane & 1) && (lane >> 1) < JC_M) out[p * (JC_M + 1) + (lane >> 1)] = (float)(v[p] * INV_SQRT_PI);
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1) {
     e_min = fminf(e_min, __shfl_xor_sync(0xffffffffu, e_min, o));
@@ -456,7 +462,7 @@ jac_far_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__ jpr
                float* __restrict__ l1_coef, CellGeom cg, const int* __restrict__ cell_idx,
                const float* __restrict__ cell_rec) {
   __shared__ LineSplit<MJF_THREADS> s_split;
-  __shared__ float s_cell[MJF_THREADS / 32][3][MJ_KF];
+  __shared__ double s_cell[MJF_THREADS / 32][3][MJ_KF];
   __shared__ __align__(16) float4 s_line[MJF_STAGES][4][MJF_THREADS];  // 64-B records as four 16-B planes
   __shared__ double s_part[MJF_THREADS / 32][MJ_NCOEF];                 // [q][16] then [q][8] per warp
 
@@ -503,8 +509,18 @@ jac_far_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__ jpr
     const int k = tid & (MJ_KF - 1);
     const float xk = k < MJ_KF / 2 ? H1 * c_jnode8[k] : -H1 * c_jnode8[MJ_KF - 1 - k];
     const float half = 0.5f * (float)cg.wp;
+    double sum[3] = {0.0, 0.0, 0.0};
     float f[3] = {0.f, 0.f, 0.f};
+    int rounds = 0;
     for (int i = tid >> 3; i < n_use; i += MJF_THREADS / 8) {
+      if (++rounds > MJF_FLUSH) {
+        rounds = 1;
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+          sum[p] += (double)f[p];
+          f[p] = 0.f;
+        }
+      }
       const int q = s_split.use[i];
       const float4* r4 = reinterpret_cast<const float4*>(rec_row + (long long)q * JC_F);
       const float D = (H1 + xk) - ((float)((long long)q * cg.wp - cg.off - c0) + half);
@@ -530,9 +546,10 @@ jac_far_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__ jpr
     }
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
-      f[p] += __shfl_xor_sync(0xffffffffu, f[p], 8);
-      f[p] += __shfl_xor_sync(0xffffffffu, f[p], 16);
-      if ((tid & 31) < MJ_KF) s_cell[warp][p][tid & 31] = f[p];
+      sum[p] += (double)f[p];
+      sum[p] += __shfl_xor_sync(0xffffffffu, sum[p], 8);
+      sum[p] += __shfl_xor_sync(0xffffffffu, sum[p], 16);
+      if ((tid & 31) < MJ_KF) s_cell[warp][p][tid & 31] = sum[p];
     }
   }
   jfar_pass<MJ_KF>(s_line, lp, jp, n_direct, [&](int i) { return split ? split_line(s_split, n_dir, i) : rng.x + i; },
@@ -542,7 +559,7 @@ jac_far_kernel(const LineF32* __restrict__ prep, const LineJac* __restrict__ jpr
     double v = 0.0;
     for (int w = 0; w < MJF_THREADS / 32; ++w) v += s_part[w][c];
     if (n_use > 0 && c >= 3 * MJ_K)
-      for (int w = 0; w < MJF_THREADS / 32; ++w) v += (double)(&s_cell[w][0][0])[c - 3 * MJ_K];
+      for (int w = 0; w < MJF_THREADS / 32; ++w) v += (&s_cell[w][0][0])[c - 3 * MJ_K];
     s_part[0][c] = v;
   }
   __syncthreads();
