@@ -522,7 +522,7 @@ adam_group_kernel(const __grid_constant__ AdamGroup grp, int n, float lr, float 
     *(float4*)(I.m + o) = m;
     *(float4*)(I.v + o) = v;
     *(float4*)(I.w + o) = w;
-    const __nv_bfloat16 h[4] = {__float2bfloat16(w.x), __float2bfloat16(w.y), __float2bfloat16(w.z), __float2bfloat16(w.w)};
+    __align__(8) const __nv_bfloat16 h[4] = {__float2bfloat16(w.x), __float2bfloat16(w.y), __float2bfloat16(w.z), __float2bfloat16(w.w)};
     if (w_bf) *(uint2*)(w_bf + o) = *(const uint2*)h;
     if (wt_bf)
 #pragma unroll
@@ -534,7 +534,7 @@ adam_group_kernel(const __grid_constant__ AdamGroup grp, int n, float lr, float 
   for (int i = threadIdx.x; i < cols * (ADAM_T / 4); i += 256) {
     const int c = i / (ADAM_T / 4), r = 4 * (i % (ADAM_T / 4));
     if (r >= rows) continue;
-    const __nv_bfloat16 h[4] = {s_t[c][r], s_t[c][r + 1], s_t[c][r + 2], s_t[c][r + 3]};
+    __align__(8) const __nv_bfloat16 h[4] = {s_t[c][r], s_t[c][r + 1], s_t[c][r + 2], s_t[c][r + 3]};
     *(uint2*)(wt_bf + (long long)(c0 + c) * I.rows + r0 + r) = *(const uint2*)h;
   }
 }
