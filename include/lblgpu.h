@@ -430,6 +430,11 @@ int lbl_stage_batch(const float* features, const float* targets, const long long
 int lbl_ensemble_gate(const float* pred, int n_mem, long long member_stride, int n_samples, int ld, int n_ch,
                       const float* ch_scale, float scale, float gate, float* mean, float* est, int* flag,
                       void* stream);
+/* The same with the error word of the members' products (device, nullable): while it is not 0 every
+ * mean and est is NaN and every flag set. */
+int lbl_ensemble_gate_checked(const float* pred, int n_mem, long long member_stride, int n_samples, int ld, int n_ch,
+                              const float* ch_scale, float scale, float gate, const int* err, float* mean, float* est,
+                              int* flag, void* stream);
 
 /* Measurement probe (no reference counterpart): `blocks` CTAs of 256 threads
  * each run 8 chains of `iters` dependent float32 FMAs, i.e.

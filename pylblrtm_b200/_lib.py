@@ -84,6 +84,7 @@ SIGNATURES = {
     "lbl_pack_inputs_bf16": (_I, [_P, _I, _I, _P, _P, _P, _I, _P, _I, _P]),
     "lbl_stage_batch": (_I, [_P, _P, _P, _L, _I, _I, _I, _P, _P, _P, _I, _P, _I, _P, _P, _P]),
     "lbl_ensemble_gate": (_I, [_P, _I, _L, _I, _I, _I, _P, _F, _F, _P, _P, _P, _P]),
+    "lbl_ensemble_gate_checked": (_I, [_P, _I, _L, _I, _I, _I, _P, _F, _F, _P, _P, _P, _P, _P]),
 }
 
 # epilogue modes of lbl_gemm_bf16

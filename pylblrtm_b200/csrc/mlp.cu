@@ -723,7 +723,7 @@ __device__ __forceinline__ void gate_channel(int n_mem, Load load, float& mu, fl
   sd = sqrtf(s2 / n_mem);
 }
 
-__device__ __forceinline__ void gate_finish(float worst, float scale, float gate, float* est, int* flag) {
+__device__ __forceinline__ void gate_finish(float worst, float scale, float gate, bool bad, float* est, int* flag) {
   for (int o = 16; o > 0; o >>= 1) worst = fmaxf(worst, __shfl_xor_sync(0xffffffffu, worst, o));
   __shared__ float part[32];
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = worst;
@@ -731,24 +731,26 @@ __device__ __forceinline__ void gate_finish(float worst, float scale, float gate
   if (threadIdx.x == 0) {
     float t = 0.f;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t = fmaxf(t, part[w]);
-    *est = t;
-    *flag = (scale * t > gate) ? 1 : 0;
+    *est = bad ? __int_as_float(0x7fffffff) : t;
+    *flag = (bad || scale * t > gate) ? 1 : 0;
   }
 }
 
 __global__ void ensemble_gate_kernel(const float* __restrict__ pred, int n_mem, long long member_stride, int ld,
                                      int n_ch, const float* __restrict__ ch_scale, float scale, float gate,
-                                     float* __restrict__ mean, float* __restrict__ est, int* __restrict__ flag) {
+                                     const int* err, float* __restrict__ mean, float* __restrict__ est,
+                                     int* __restrict__ flag) {
+  const bool bad = err && *err != 0;
   const int b = blockIdx.x;
   float worst = 0.0f;
   for (int c = threadIdx.x; c < n_ch; c += blockDim.x) {
     const float* col = pred + (long long)b * ld + c;
     float mu, sd;
     gate_channel(n_mem, [&](int m) { return col[m * member_stride]; }, mu, sd);
-    mean[(long long)b * n_ch + c] = mu;
+    mean[(long long)b * n_ch + c] = bad ? __int_as_float(0x7fffffff) : mu;
     worst = fmaxf(worst, ch_scale ? ch_scale[c] * sd : sd);
   }
-  gate_finish(worst, scale, gate, est + b, flag + b);
+  gate_finish(worst, scale, gate, bad, est + b, flag + b);
 }
 
 // The same for NM members held in registers, four channels per thread and load (n_ch, ld and
@@ -758,11 +760,13 @@ __global__ void ensemble_gate_kernel(const float* __restrict__ pred, int n_mem, 
 template <int NM>
 __global__ void __launch_bounds__(256)
 ensemble_gate4_kernel(const float4* __restrict__ pred, long long member_stride4, int ld4, int n_ch4,
-                      const float* __restrict__ ch_scale, float scale, float gate, float4* __restrict__ mean,
-                      float* __restrict__ est, int* __restrict__ flag) {
+                      const float* __restrict__ ch_scale, float scale, float gate, const int* err,
+                      float4* __restrict__ mean, float* __restrict__ est, int* __restrict__ flag) {
   dependency_trigger();
   dependency_wait();
   const int b = blockIdx.x;
+  const bool bad = err && *err != 0;
+  const float nan = __int_as_float(0x7fffffff);
   float worst = 0.0f;
   for (int c = threadIdx.x; c < n_ch4; c += blockDim.x) {
     const float4* col = pred + (long long)b * ld4 + c;
@@ -779,9 +783,9 @@ ensemble_gate4_kernel(const float4* __restrict__ pred, long long member_stride4,
       gate_channel(NM, [&](int m) { return v[m][i]; }, mu[i], sd);
       worst = fmaxf(worst, ch_scale ? ch_scale[4 * c + i] * sd : sd);
     }
-    mean[(long long)b * n_ch4 + c] = make_float4(mu[0], mu[1], mu[2], mu[3]);
+    mean[(long long)b * n_ch4 + c] = bad ? make_float4(nan, nan, nan, nan) : make_float4(mu[0], mu[1], mu[2], mu[3]);
   }
-  gate_finish(worst, scale, gate, est + b, flag + b);
+  gate_finish(worst, scale, gate, bad, est + b, flag + b);
 }
 
 }  // namespace lbl
@@ -1118,9 +1122,9 @@ extern "C" int lbl_stage_batch(const float* features, const float* targets, cons
   return lbl_check_launch("lbl_stage_batch");
 }
 
-extern "C" int lbl_ensemble_gate(const float* pred, int n_mem, long long member_stride, int n_samples, int ld,
-                                 int n_ch, const float* ch_scale, float scale, float gate, float* mean, float* est,
-                                 int* flag, void* stream) {
+extern "C" int lbl_ensemble_gate_checked(const float* pred, int n_mem, long long member_stride, int n_samples, int ld,
+                                         int n_ch, const float* ch_scale, float scale, float gate, const int* err,
+                                         float* mean, float* est, int* flag, void* stream) {
   if (!pred || !mean || !est || !flag || n_mem < 1 || n_samples < 1 || n_ch < 1 || ld < n_ch ||
       (n_mem > 1 && member_stride < (long long)n_samples * ld))
     return lbl_set_error(LBL_EINVAL, "lbl_ensemble_gate: bad arguments");
@@ -1128,7 +1132,7 @@ extern "C" int lbl_ensemble_gate(const float* pred, int n_mem, long long member_
   const bool vec = n_ch % 4 == 0 && ld % 4 == 0 && member_stride % 4 == 0 && ((uintptr_t)pred | (uintptr_t)mean) % 16 == 0;
   auto vec_launch = [&](auto nm) {
     launch_dependent(ensemble_gate4_kernel<decltype(nm)::value>, dim3((unsigned)n_samples), 256, 0, st, (const float4*)pred,
-                     member_stride / 4, ld / 4, n_ch / 4, ch_scale, scale, gate, (float4*)mean, est, flag);
+                     member_stride / 4, ld / 4, n_ch / 4, ch_scale, scale, gate, err, (float4*)mean, est, flag);
   };
   if (vec && n_mem == 2) vec_launch(std::integral_constant<int, 2>());
   else if (vec && n_mem == 3) vec_launch(std::integral_constant<int, 3>());
@@ -1137,7 +1141,14 @@ extern "C" int lbl_ensemble_gate(const float* pred, int n_mem, long long member_
   else if (vec && n_mem == 6) vec_launch(std::integral_constant<int, 6>());
   else if (vec && n_mem == 8) vec_launch(std::integral_constant<int, 8>());
   else
-    ensemble_gate_kernel<<<n_samples, 256, 0, st>>>(pred, n_mem, member_stride, ld, n_ch, ch_scale, scale, gate, mean,
-                                                    est, flag);
+    ensemble_gate_kernel<<<n_samples, 256, 0, st>>>(pred, n_mem, member_stride, ld, n_ch, ch_scale, scale, gate, err,
+                                                    mean, est, flag);
   return lbl_check_launch("lbl_ensemble_gate");
+}
+
+extern "C" int lbl_ensemble_gate(const float* pred, int n_mem, long long member_stride, int n_samples, int ld,
+                                 int n_ch, const float* ch_scale, float scale, float gate, float* mean, float* est,
+                                 int* flag, void* stream) {
+  return lbl_ensemble_gate_checked(pred, n_mem, member_stride, n_samples, ld, n_ch, ch_scale, scale, gate, nullptr, mean,
+                                   est, flag, stream);
 }

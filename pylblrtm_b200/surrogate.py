@@ -201,6 +201,11 @@ class _Workspace:
         self.err = torch.zeros((1,), dtype=torch.int32, device=dev)
 
 
+def _raise_on_timeout(err) -> None:
+    if int(err.item()) != 0:
+        raise RuntimeError("lbl_gemm_bf16: a tensor-core pipeline wait timed out")
+
+
 class MLP:
     """n_in -> hidden x depth (GELU) -> n_out (sigmoid) in BF16 with float32 accumulation.
 
@@ -314,16 +319,18 @@ class MLP:
             self._ws[key] = _Workspace(self, batch, train)
         return self._ws[key]
 
-    def _gemm(self, map_a, map_b, m, n, k, ep, ws, stream, n_split=1):
+    def _gemm(self, map_a, map_b, m, n, k, ep, err, stream, n_split=1):
         _lib.call("lbl_gemm_bf16", map_a.addr, map_b.addr, m, n, k, n_split, ctypes.addressof(ep),
-                  ws.err.data_ptr(), stream)
+                  err.data_ptr(), stream)
         self.launches += 1
 
-    def _forward(self, ws: _Workspace, stream, train: bool, out=None, packed: bool = False) -> None:
+    def _forward(self, ws: _Workspace, stream, train: bool, out=None, packed: bool = False, err=None) -> None:
         """Forward pass; inference writes the sigmoid output to ``out`` (float32
         [B, n_out padded], row stride n_out padded) or to the workspace. ``packed``: the
-        workspace already holds the standardised inputs."""
+        workspace already holds the standardised inputs. ``err``: the products' error word
+        (the workspace's)."""
         B = ws.batch
+        err = ws.err if err is None else err
         L = len(self.dims)
         if not packed:
             _lib.call("lbl_pack_inputs_bf16", ws.raw.data_ptr(), B, self.n_in, self.mean.data_ptr(),
@@ -350,7 +357,7 @@ class MLP:
                     ep.loss = ws.loss.data_ptr()
                 else:
                     ep.out_f32, ep.ld_f32 = (ws.out if out is None else out).data_ptr(), n
-            self._gemm(ws.map_x[li], self.map_w[li], B, n, k, ep, ws, stream)
+            self._gemm(ws.map_x[li], self.map_w[li], B, n, k, ep, err, stream)
 
     def _backward(self, ws: _Workspace, stream) -> None:
         B = ws.batch
@@ -362,7 +369,7 @@ class MLP:
             ep[1].mode = _lib.GEMM_F32
             ep[1].out_f32, ep[1].ld_f32, ep[1].split_stride = ws.dw[li].data_ptr(), k, n * k
             if li == 0:
-                self._gemm(ws.map_dzt[0], ws.map_xt[0], n, k, B, ep[1], ws, stream, n_split=s)
+                self._gemm(ws.map_dzt[0], ws.map_xt[0], n, k, B, ep[1], ws.err, stream, n_split=s)
                 break
             ep[0].mode = _lib.GEMM_DGELU
             ep[0].z_in, ep[0].ld_zin = ws.z[li - 1].data_ptr(), k
@@ -395,8 +402,7 @@ class MLP:
         self.launches += -(-len(items) // 16)
 
     def _check(self, ws: _Workspace) -> None:
-        if int(ws.err.item()) != 0:
-            raise RuntimeError("lbl_gemm_bf16: a tensor-core pipeline wait timed out")
+        _raise_on_timeout(ws.err)
 
     def train_step(self, raw, target, lr: Optional[float] = None, check: bool = False):
         """One Adam step on a batch (device tensors raw [B, n_in], target [B, n_out] float32).
@@ -516,6 +522,9 @@ class GatedSurrogate:
         self.deterministic = bool(deterministic)      # of the engine fallback
         self.torch = members[0].torch
         self.launches = 0
+        # the error word of the members' products: the gate turns results into NaN and sets every
+        # flag while it is not 0, check() raises
+        self.err = self.torch.tensor([0], dtype=self.torch.int32, device=members[0].dev)
         self.ch_scale = None
         if ch_scale is not None:
             w = np.ascontiguousarray(ch_scale, dtype=np.float32).reshape(-1)
@@ -523,8 +532,13 @@ class GatedSurrogate:
                 raise ValueError(f"ch_scale needs {members[0].n_out} values, got {w.size}")
             self.ch_scale = self.torch.as_tensor(w, device=members[0].dev)
 
+    def check(self) -> None:
+        """Raise if a product of an earlier prediction failed (waits for the device)."""
+        _raise_on_timeout(self.err)
+
     def predictions(self, raw):
-        """Every member's channel predictions [n_members, B, n_out] (device)."""
+        """Every member's channel predictions [n_members, B, n_out] (device); :meth:`check` tells
+        whether they are complete."""
         pred, B, _ = self._members(raw)
         return pred[:, :B, :self.members[0].n_out]
 
@@ -551,7 +565,7 @@ class GatedSurrogate:
             widths = (ctypes.c_int * (len(net0.dims) + 1))(net0.dims[0][0], *[n for _, n in net0.dims])
             _lib.call("lbl_ensemble_forward", x.data_ptr(), B, net0.n_in, (ctypes.c_void_p * len(items))(*items),
                       (ctypes.c_void_p * len(layers))(*layers), len(nets), len(net0.dims), widths, Bp, net0.n_out,
-                      pred.data_ptr(), Bp * n_pad, wss[0].err.data_ptr(), stream)
+                      pred.data_ptr(), Bp * n_pad, self.err.data_ptr(), stream)
             self.launches = -(-len(nets) // 16) + len(net0.dims) * -(-len(nets) // 8)
             for net in nets:
                 net.launches = 1 + len(net0.dims)
@@ -562,12 +576,13 @@ class GatedSurrogate:
             ws.raw[:B].copy_(raw)
             if Bp > B:
                 ws.raw[B:].zero_()
-            net._forward(ws, stream, False, out=pred[m])
+            net._forward(ws, stream, False, out=pred[m], err=self.err)
             self.launches += net.launches
         return pred, B, stream
 
     def ensemble(self, raw):
-        """(mean [B, n_out], est [B], flag [B] bool) on the device."""
+        """(mean [B, n_out], est [B], flag [B] bool) on the device; NaN and flagged throughout when a
+        member's product failed."""
         torch = self.torch
         net0 = self.members[0]
         pred, B, stream = self._members(raw)
@@ -575,9 +590,9 @@ class GatedSurrogate:
         mean = torch.empty((B, net0.n_out), dtype=torch.float32, device=net0.dev)
         est = torch.empty((B,), dtype=torch.float32, device=net0.dev)
         flag = torch.empty((B,), dtype=torch.int32, device=net0.dev)
-        _lib.call("lbl_ensemble_gate", pred.data_ptr(), len(self.members), Bp * n_pad, B, n_pad, net0.n_out,
-                  _lib.ptr(self.ch_scale), self.scale, self.gate, mean.data_ptr(), est.data_ptr(), flag.data_ptr(),
-                  stream)
+        _lib.call("lbl_ensemble_gate_checked", pred.data_ptr(), len(self.members), Bp * n_pad, B, n_pad, net0.n_out,
+                  _lib.ptr(self.ch_scale), self.scale, self.gate, self.err.data_ptr(), mean.data_ptr(), est.data_ptr(),
+                  flag.data_ptr(), stream)
         self.launches += 1
         return mean, est, flag.bool()
 
@@ -595,6 +610,7 @@ class GatedSurrogate:
         t0 = time.perf_counter()
         mean, est, flag = self.ensemble(raw)
         flag_h = flag.cpu().numpy()
+        self.check()
         t1 = time.perf_counter()
         idx = np.flatnonzero(flag_h)
         if idx.size:
@@ -622,6 +638,7 @@ def calibrate_gate(gs: "GatedSurrogate", raw, reference: np.ndarray, target: flo
     pred = gs.predictions(torch.as_tensor(raw, device=gs.members[0].dev))
     mean = pred.mean(0)
     spread = pred.std(0, unbiased=False).cpu().numpy()
+    gs.check()
     err_c = np.abs(mean.cpu().numpy() - np.asarray(reference, dtype=np.float32))
     err = err_c.max(1)
     fitted = channel_weights(spread, err_c)
