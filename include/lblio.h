@@ -61,7 +61,7 @@ long long lbl_count_band(const double* nu0, const double* shift, const int* gid,
 
 /* lbl_line_pairs that also lists the lines inside the band mask: *n_band of them, their
  * positions in the list (band_line) and pairs (band_pair), in input order; both arrays have
- * room for n entries. Runs on up to eight threads of its own for long lists. */
+ * room for n entries. Long lists are scanned on up to six threads. */
 int lbl_band_scan(const int* mol, const int* iso, const double* nu0, const double* shift, long long n,
                   double lo_edge, double hi_edge, double p_max, int max_pairs, int* pair_mol, int* pair_iso,
                   long long* pair_band, int* n_pairs, int* band_line, int* band_pair, long long* n_band,

@@ -3,8 +3,8 @@
 ``AtmosphericProfile`` validates levels exactly like ``atmosphere.py:63-100``.
 ``build_layers`` is kept on the host for API compatibility
 (``atmosphere.py:110-141``); the forward engine builds the same layers on the
-device (``lbl_build_layers``) with the same operation order, and the tests check
-the two agree bit for bit.
+device (``lbl_layer_setup``; ``lbl_build_layers`` alone) with the same operation order,
+and the tests check that they agree bit for bit.
 """
 
 from __future__ import annotations

@@ -755,8 +755,10 @@ __global__ void ensemble_gate_kernel(const float* __restrict__ pred, int n_mem, 
 
 // The same for NM members held in registers, four channels per thread and load (n_ch, ld and
 // member_stride multiples of 4, 16-byte aligned rows): each prediction is read once, with
-// NM 16-byte loads in flight per thread. HBM-bound; 20,000 samples x 2,000 channels x 4
-// members: 0.122 against 0.237 ms of the scalar kernel above, which serves the other shapes.
+// NM 16-byte loads in flight per thread. HBM-bound; 20,000 samples x 2,000 channels, this and the
+// scalar kernel above: 76 and 224 us for 2 members, 104 and 236 for 3, 122 and 199 for 4, 147 and
+// 269 for 5, 172 and 333 for 6, 217 and 300 for 8. Seven members and more than eight are not
+// compiled here (no configuration has them) and take the scalar kernel: 349 us for 7, 375 for 9.
 template <int NM>
 __global__ void __launch_bounds__(256)
 ensemble_gate4_kernel(const float4* __restrict__ pred, long long member_stride4, int ld4, int n_ch4,

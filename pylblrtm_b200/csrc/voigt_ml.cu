@@ -342,7 +342,7 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
   const bool split = split_lines<MF_THREADS, CELL_F, CELL_M>(s_split, cg, cell_idx, rec_row, rng, t0, t1, c0, H1,
                                                              cutoff, step, n_use, n_dir, n_direct);
   const bool cells = n_use > 0;
-  if (cells) {                                             // thread: node tid % 8 of cells tid / 8, + 32, ...
+  if (cells) {                                             // thread: node tid % 8 of cells tid / 8, + 8, ...
     const int k = tid & (ML_KF - 1);
     const float xk = k < ML_KF / 2 ? H1 * c_node8[k] : -H1 * c_node8[ML_KF - 1 - k];
     const float half = 0.5f * (float)cg.wp;
@@ -484,8 +484,9 @@ tau_far_kernel(const LineF32* __restrict__ prep, int n_lines, const int2* __rest
 //    warp's float64 node sums;
 //  * level 3: each lane evaluates the line at its own 8 points, two per instruction
 //    (fma.rn.f32x2: whole spectrum 8.65 -> 8.05 ms, the series at the end in pairs too 8.00;
-//    pairs of level-2 nodes cost spills, 8.09), by the clamped five-term form, or by the two-term form when the line is far from every point of
-//    the sub-chunk (|z|^2 >= FAR_Z2 there);
+//    pairs of level-2 nodes cost spills, 8.09), by the clamped five-term form, or by the
+//    two-term form when the line is far from every point of the sub-chunk (|z|^2 >= FAR_Z2
+//    there);
 //  * near zones: the near points of the warp's level-3 lines inside its sub-chunk form
 //    an item space (middles, where the float64 core may apply, then tails); lanes take
 //    consecutive items, find their line by a shuffle search over a group of 32 lines

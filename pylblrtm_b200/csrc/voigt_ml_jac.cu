@@ -50,7 +50,8 @@ constexpr int MJ_NCOEF = 3 * (MJ_K + MJ_KF);       // level-1 coefficients per (
 // Level 1 is latency-bound once its far lines come as cells: small CTAs cover each other's
 // waits. 200 cm^-1, 60 layers, 26,000 lines on B200: every line by itself 1,235 us (1,100 with
 // the transposed flush); with cells and CTAs of 256, 128 and 64 threads 551, 393 and 337 us
-// (plus 66 us for the moments); 6 instead of 8 CTAs per SM 385 us.
+// (plus 97 us for the moments, 66 with float32 sums across the lanes, which put the error of far
+// wings at 1.4 times the line-by-line error instead of 1.17); 6 instead of 8 CTAs per SM 385 us.
 constexpr int MJF_THREADS = 64;                    // lines per round of jac_far_kernel
 constexpr int MJF_CTAS = 8;                        // per SM
 constexpr int MJF_STAGES = 2;                      // rounds of line records in flight per thread

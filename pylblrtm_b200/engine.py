@@ -2,14 +2,14 @@
 
 One call of :func:`optical_depth` runs, on the current CUDA stream:
 
-1. ``lbl_build_layers``  levels -> layers (or an upload of host layers)
-2. ``lbl_layer_groups``  per (layer, line group) pressures, column, Q(296)/Q(T)
-3. ``lbl_sort_lines``    reference band mask + sort by centre
-4. ``lbl_gather_lines``  sorted line records
-5. ``lbl_tile_ranges``   candidate lines of every reference tile
-6. ``lbl_line_prep_*``   per (layer, line) strengths and widths
-7. ``lbl_tau_tiles_*``   Voigt sums x R(nu, T) -> od[layer, nu]
-8. ``lbl_layer_sum_exp_*`` (optional) column tau and exp(-tau/mu)
+1. ``lbl_layer_setup``    levels -> layers (or the uploaded host layers), and per (layer,
+   line group) pressures, column, Q(296)/Q(T)
+2. ``lbl_sort_gather``    reference band mask, sort by centre, sorted line records
+3. ``lbl_line_ranges``    candidate lines of every reference tile
+4. ``lbl_line_prep_*``    per (layer, line) strengths and widths
+5. ``lbl_line_cells``     (multi-level float32 sums on long grids) far lines by cells
+6. ``lbl_tau_tiles_*``    Voigt sums x R(nu, T) -> od[layer, nu]
+7. ``lbl_layer_sum_exp_*`` (optional) column tau and exp(-tau/mu)
 
 Host work is limited to what the reference does once per call in Python: the
 (mol, iso) group selection with its warnings and errors

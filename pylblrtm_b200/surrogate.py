@@ -9,11 +9,14 @@ box-averaging), so the network learns this library's own forward model.
 Everything numeric runs in ``liblblgpu.so`` (include/lblgpu.h):
   * ``lbl_gemm_bf16`` -- BF16 tensor-core GEMM (tcgen05, TMA, float32 accumulators in
     tensor memory) with fused epilogues: bias + GELU (forward), bias + sigmoid + MSE
-    gradient (output layer), GELU' (backward), float32 split-K partials (weight grads);
-  * ``lbl_adam_step`` -- Adam on float32 master weights that refreshes the bf16
-    weights and their transposes; ``lbl_rowsum_bf16`` -- bias gradients;
-  * ``lbl_pack_inputs_bf16`` -- standardisation; ``lbl_ensemble_gate`` -- ensemble
-    mean, spread and gate flag.
+    gradient (output layer), GELU' (backward), float32 split-K partials (weight grads)
+    (``lbl_gemm_bf16_pair``: a layer's weight and input gradients in one launch);
+  * ``lbl_adam_group`` -- Adam on float32 master weights that refreshes the bf16
+    weights and their transposes; ``lbl_rowsum_group`` -- bias gradients;
+  * ``lbl_stage_batch`` -- gathered and standardised training batches;
+    ``lbl_pack_inputs_bf16`` -- standardisation of other inputs;
+  * ``lbl_ensemble_forward`` -- all members of one architecture, layer by layer;
+    ``lbl_ensemble_gate_checked`` -- ensemble mean, spread and gate flag.
 Every GEMM is "A . B^T" with both operands K-contiguous, so the backward pass keeps
 transposed copies: W and W^T, activations X and X^T, output gradients dZ and dZ^T.
 Widths are padded to multiples of 128 (inputs 61 -> 128, outputs 2000 -> 2048); the

@@ -96,3 +96,34 @@ def test_small_and_negative_widths(tile_pts, width, monkeypatch):
     general = restate.optical_depth(nu, sd.lines, sd.tips, sd.molar_masses, p, t, v, c, cutoff, tile)
     at = near < 3.0
     assert np.max(err[0, at]) <= 1e-12 + np.max(np.abs(general - ref)[0, at] / scale[0, at])
+
+
+# One line, 24 to 700 Doppler units away, summed point by point: one reciprocal and the series per value, in
+# the wings of small, ordinary and large y. The reference sums the asymptotic series in long double (wofz
+# carries 5e-15 at y = 36). Ratios to the median take the line's strength out; what is left is a dozen
+# roundings of 1.1e-16 (an uncorrected estimate of 1/|z|^2 would show 1e-6, one Newton step 1e-12).
+@pytest.mark.gpu
+@pytest.mark.parametrize("width", [1e-4, 0.02, 1.0])
+def test_reciprocal_of_the_wings(width, monkeypatch):
+    from pylblrtm_b200 import engine, synthetic
+
+    def series_voigt(nu, centers, doppler, lorentz):
+        z = (restate.SQRT_LN2 * ((nu[:, None] - centers) + 1j * lorentz) / doppler).astype(np.clongdouble)
+        u, s = 1 / (z * z), np.zeros_like(z)
+        for k in range(30, -1, -1):                          # (2k - 1)!! / 2^k z^-2k by Horner
+            s = 1 + (k + np.longdouble(0.5)) * u * s
+        return (-(s / z).imag / np.sqrt(np.longdouble(np.pi))).astype(np.float64) * (restate.VOIGT_K / doppler)
+
+    monkeypatch.setattr(restate, "voigt", series_voigt)
+    sd = synthetic.co2_band(1, 719.9999, 720.0001, seed=3)
+    for k in ("g_air", "g_self"):
+        sd.lines[k] = np.full(1, width)
+    prof = synthetic.logp_profile(2)
+    lo, step, cutoff = 720.02, 5e-4, 1.0
+    hi, tile = lo + 999.5 * step, 8.25 * step
+    p, t, v, c = restate.build_layers(prof.pressure_hpa, prof.temperature_k, prof.vmr)
+    ref = restate.optical_depth(restate.grid(lo, hi, step), sd.lines, sd.tips, sd.molar_masses, p, t, v, c, cutoff, tile)
+    res = engine.optical_depth(sd, engine.layer_input_from_profile(prof), engine.make_grid(lo, hi, step, tile), cutoff,
+                               precision="fp64")
+    ratio = (res.od[0].cpu().numpy() / ref)[0]
+    assert np.max(np.abs(ratio / np.median(ratio) - 1.0)) <= 3e-15
